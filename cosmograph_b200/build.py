@@ -30,15 +30,17 @@ NVCC = os.environ.get("NVCC", "/usr/local/cuda/bin/nvcc")
 ARCH = ["-gencode", "arch=compute_100a,code=sm_100a"]
 COMMON = ["-std=c++17", "-O3", "-lineinfo", "-Xcompiler", "-fPIC", *ARCH, f"-I{INCLUDE}", f"-I{CSRC}"]
 
-# (object name, source, extra flags)
+_EXACT = ["--fmad=false", "-DCG_VARIANT_NS=exact", "-DCG_REFERENCE_ORDER=1"]
+_FAST = ["--fmad=true", "-DCG_VARIANT_NS=fast"]
+# (object name, source, extra flags); the substep kernels one unit per stencil
+# order and variant, the slowest to compile first
 UNITS = [
-    ("stage_exact.o", "cg_stage_inst.cu", ["--fmad=false", "-DCG_VARIANT_NS=exact", "-DCG_REFERENCE_ORDER=1"]),
-    ("stage_fast.o", "cg_stage_inst.cu", ["--fmad=true", "-DCG_VARIANT_NS=fast"]),
-    ("stage_exact_z4c.o", "cg_stage_inst.cu",
-     ["--fmad=false", "-DCG_VARIANT_NS=exact", "-DCG_REFERENCE_ORDER=1", "-DCG_Z4C_UNIT=1"]),
-    ("stage_fast_z4c.o", "cg_stage_inst.cu", ["--fmad=true", "-DCG_VARIANT_NS=fast", "-DCG_Z4C_UNIT=1"]),
-    ("stage_exact_shift.o", "cg_stage_inst.cu",
-     ["--fmad=false", "-DCG_VARIANT_NS=exact", "-DCG_REFERENCE_ORDER=1", "-DCG_SHIFT_UNIT=1"]),
+    *[(f"stage_{name}_o{o}.o", "cg_stage_inst.cu", [*flags, f"-DCG_ORDER={o}"])
+      for name, flags in (("exact_shift", [*_EXACT, "-DCG_SHIFT_UNIT=1"]), ("exact", _EXACT), ("fast", _FAST),
+                          ("exact_z4c", [*_EXACT, "-DCG_Z4C_UNIT=1"]), ("fast_z4c", [*_FAST, "-DCG_Z4C_UNIT=1"]))
+      for o in (8, 2, 4, 6)],
+    ("stage_exact.o", "cg_stage_inst.cu", _EXACT),
+    ("stage_fast.o", "cg_stage_inst.cu", _FAST),
     ("abi.o", "cg_abi.cu", []),
     ("noalloc.o", "cg_noalloc.cu", []),
     ("peak.o", "cg_peak.cu", []),
@@ -75,7 +77,7 @@ def build(force: bool = False, verbose: bool = False) -> Path:
             sys.stderr.write(r.stderr)
 
     if jobs:
-        with ThreadPoolExecutor(max_workers=len(jobs)) as ex:
+        with ThreadPoolExecutor(max_workers=min(len(jobs), os.cpu_count() or 1)) as ex:
             list(ex.map(run, jobs))
     if force or jobs or not LIB.exists() or LIB.stat().st_mtime < max(o.stat().st_mtime for o in objs):
         tmp = LIB.with_suffix(".so.tmp")

@@ -89,20 +89,11 @@ cudaError_t launch_init(const BoxDev& b, const StageBg& bg, cudaStream_t st);
 // (10 arrays of pts) into cvals, 27 partial results per CTA into cpart
 cudaError_t launch_constraints(const BoxDev& b, const StageBg& bg, double* cvals, double* cpart, cudaStream_t st);
 int constraint_blocks(const BoxDev& b);
-// the Z4c instantiations (cg_stage_inst.cu built with -DCG_Z4C_UNIT=1)
-cudaError_t launch_stage_z4c(const BoxDev& b, const StageBg& bg, int stage, cudaStream_t st);
-cudaError_t launch_constraints_z4c(const BoxDev& b, const StageBg& bg, double* cvals, double* cpart, cudaStream_t st);
-// the shift instantiations (cg_stage_inst.cu built with -DCG_SHIFT_UNIT=1; the
-// parity build only)
-cudaError_t launch_stage_shift(const BoxDev& b, const StageBg& bg, int stage, cudaStream_t st);
 }  // namespace exact
 namespace fast {
 void make_tile_maps(BoxDev& b);
 cudaError_t launch_stage(const BoxDev& b, const StageBg& bg, int stage, cudaStream_t st);
 cudaError_t launch_init(const BoxDev& b, const StageBg& bg, cudaStream_t st);
-cudaError_t launch_stage_z4c(const BoxDev& b, const StageBg& bg, int stage, cudaStream_t st);
-cudaError_t launch_constraints_z4c(const BoxDev& b, const StageBg& bg, double* cvals, double* cpart, cudaStream_t st);
-cudaError_t launch_stage_shift(const BoxDev& b, const StageBg& bg, int stage, cudaStream_t st);
 }  // namespace fast
 
 // One launch for substep `stage` of every box of an FP64 group (table: device

@@ -3,6 +3,8 @@
 // Compiled twice: with -DCG_VARIANT_NS=exact and --fmad=false (the parity
 // build: every product and sum rounds separately, as in the reference's
 // strict build), and with -DCG_VARIANT_NS=fast and --fmad=true.
+#include <type_traits>
+
 #include "cg_internal.h"
 #include "cg_stage.cuh"
 
@@ -11,17 +13,23 @@
 #endif
 
 // Built a second time with -DCG_Z4C_UNIT=1: the Z4c-damping instantiations of
-// the substep and constraint kernels (launch_stage_z4c, launch_constraints_z4c)
-// in a translation unit of their own, so that the two compile in parallel.
+// the substep and constraint kernels in a translation unit of their own, so
+// that the two compile in parallel.
 #ifndef CG_Z4C_UNIT
 #define CG_Z4C_UNIT 0
 #endif
 // Built with -DCG_SHIFT_UNIT=1 (parity build only): the shift instantiations
-// of the substep kernel (launch_stage_shift), Kreiss-Oliger compiled in.
+// of the substep kernel, Kreiss-Oliger compiled in.
 #ifndef CG_SHIFT_UNIT
 #define CG_SHIFT_UNIT 0
 #endif
 #define CG_AUX_UNIT (CG_Z4C_UNIT || CG_SHIFT_UNIT)
+// Each of these is built once per stencil order with -DCG_ORDER=2, 4, 6, 8
+// (the kernels of that order), and once without (order 0): the order-free
+// step-initialisation kernel and the choice of the order at a launch.
+#ifndef CG_ORDER
+#define CG_ORDER 0
+#endif
 
 namespace cg {
 namespace CG_VARIANT_NS {
@@ -29,7 +37,238 @@ namespace CG_VARIANT_NS {
 constexpr bool kZ4cUnit = CG_Z4C_UNIT != 0;
 constexpr bool kShiftUnit = CG_SHIFT_UNIT != 0;
 
+// the launchers of one stencil order, instantiated in that order's unit
+// (VARIANT: 0 plain, 1 Z4c, 2 the shift)
+constexpr int kUnit = kZ4cUnit ? 1 : (kShiftUnit ? 2 : 0);
+template <int O, int VARIANT>
+cudaError_t stage_of_order(const BoxDev& b, const StageBg& bg, int stage, cudaStream_t st);
+template <int O, int VARIANT>
+cudaError_t constraints_of_order(const BoxDev& b, const StageBg& bg, double* cvals, double* cpart, cudaStream_t st);
+template <int O>
+cudaError_t group_of_order(const GroupBox* table, const GroupBg& gb, int matter, int stage, int grid, cudaStream_t st);
+template <int O>
+int ctas_of_order(int matter);
+template <int O>
+bool maps_of_order(BoxDev& b);
+
+namespace {
+dim3 stage_block() { return dim3(kBZ, kBY, kBX); }
+// bricks of the points a substep updates: x-slab boxes skip their ghost planes
+dim3 stage_grid(const BoxDev& b) {
+  return dim3((b.nz + kBZ - 1) / kBZ, (b.ny + kBY - 1) / kBY, (b.nx - 2 * b.xg + kBX - 1) / kBX);
+}
+}  // namespace
+
+#if CG_ORDER
+// ---- the kernels of one stencil order -----------------------------------------
+namespace {
+template <int O, int M>
+cudaError_t go_stage(const BoxDev& b, const StageBg& bg, int stage, cudaStream_t st) {
+  StagePtrs P{};
+  P.kavg = b.kavg;
+  P.p = b.P;
+  P.f = b.F;
+  P.status = b.status;
+  switch (stage) {
+    case 1: P.in = b.X; P.prev = nullptr; P.out = b.Y; P.fp_in = b.FP0; P.fp_out = b.FP1; break;
+    case 2: P.in = b.Y; P.prev = b.X; P.out = b.X; P.fp_in = b.FP1; P.fp_out = b.FP0; break;
+    case 3: P.in = b.X; P.prev = b.Y; P.out = b.Y; P.fp_in = b.FP0; P.fp_out = b.FP1; break;
+    default: P.in = b.Y; P.prev = b.X; P.out = b.P; P.norm = b.X; P.fp_in = b.FP1; P.fp_out = b.FP0; break;
+  }
+  BoxGeom geo{b.nx, b.ny, b.nz, b.pts, b.xg / kBX};
+  const CUtensorMap& map = (stage == 1 || stage == 3) ? b.mapX : b.mapY;  // the substep's input
+  FluxMaps fm;
+  const CUtensorMap* fsrc = (stage == 1 || stage == 3) ? b.fmap0 : b.fmap1;
+  for (int a = 0; a < 3; ++a) fm.m[a] = fsrc[a];
+  constexpr bool Z = kZ4cUnit;
+  constexpr size_t smem = stage_smem<O, M, kEvolve, Z>();
+  if constexpr (kShiftUnit) {
+    // one instantiation per order and matter; the dissipation is switched at run time
+    static bool configured_shift = false;
+    if (!configured_shift) {
+      cudaError_t e = cudaFuncSetAttribute(stage_kernel<O, M, kEvolve, true, false, true>,
+                                           cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+      if (e != cudaSuccess) return e;
+      configured_shift = true;
+    }
+    stage_kernel<O, M, kEvolve, true, false, true><<<stage_grid(b), stage_block(), smem, st>>>(
+        geo, b.ph, bg, P, stage, map, b.tma, fm, b.fmaps);
+    return cudaGetLastError();
+  } else {
+    if constexpr (O == 2 || O == 8) {
+      if (b.ph.ko_coeff != 0.0) {  // Kreiss-Oliger dissipation: its own instantiation
+        static bool configured_ko = false;
+        if (!configured_ko) {
+          cudaError_t e = cudaFuncSetAttribute(stage_kernel<O, M, kEvolve, true, Z>,
+                                               cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+          if (e != cudaSuccess) return e;
+          configured_ko = true;
+        }
+        stage_kernel<O, M, kEvolve, true, Z><<<stage_grid(b), stage_block(), smem, st>>>(geo, b.ph, bg, P, stage, map,
+                                                                                         b.tma, fm, b.fmaps);
+        return cudaGetLastError();
+      }
+    }
+    static bool configured = false;  // per instantiation
+    if (!configured) {
+      cudaError_t e =
+          cudaFuncSetAttribute(stage_kernel<O, M, kEvolve, false, Z>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+      if (e != cudaSuccess) return e;
+      configured = true;
+    }
+    stage_kernel<O, M, kEvolve, false, Z><<<stage_grid(b), stage_block(), smem, st>>>(geo, b.ph, bg, P, stage, map,
+                                                                                      b.tma, fm, b.fmaps);
+    return cudaGetLastError();
+  }
+}
+template <int O>
+cudaError_t go_stage_m(const BoxDev& b, const StageBg& bg, int stage, cudaStream_t st) {
+  switch (b.matter) {
+    case kDust: return go_stage<O, kDust>(b, bg, stage, st);
+    case kScalar: return go_stage<O, kScalar>(b, bg, stage, st);
+#if !CG_SHIFT_UNIT  // static matter has no shift (cg_create rejects it)
+    case kStaticMatter: return go_stage<O, kStaticMatter>(b, bg, stage, st);
+#endif
+    default: return go_stage<O, kVacuum>(b, bg, stage, st);
+  }
+}
+
+#if CG_REFERENCE_ORDER && !CG_SHIFT_UNIT  // constraint statistics: the parity build's arithmetic; shift boxes take the plain kernels
+template <int O, int M>
+cudaError_t go_constraints(const BoxDev& b, const StageBg& bg, double* cvals, double* cpart, cudaStream_t st) {
+  StagePtrs P{};
+  P.in = b.X;
+  P.p = b.P;
+  P.fp_in = b.FP0;
+  P.status = b.status;
+  P.kavg = b.kavg;
+  P.cvals = cvals;
+  P.cpart = cpart;
+  BoxGeom geo{b.nx, b.ny, b.nz, b.pts, b.xg / kBX};
+  constexpr bool Z = kZ4cUnit;
+  constexpr size_t smem = stage_smem<O, M, kConstraints, Z>();
+  static bool configured = false;
+  if (!configured) {
+    cudaError_t e = cudaFuncSetAttribute(stage_kernel<O, M, kConstraints, false, Z>,
+                                         cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (e != cudaSuccess) return e;
+    configured = true;
+  }
+  FluxMaps fm{};
+  stage_kernel<O, M, kConstraints, false, Z><<<stage_grid(b), stage_block(), smem, st>>>(geo, b.ph, bg, P, 1, b.mapX,
+                                                                                         b.tma, fm, 0);
+  return cudaGetLastError();
+}
+
+template <int O>
+cudaError_t go_constraints_m(const BoxDev& b, const StageBg& bg, double* cvals, double* cpart, cudaStream_t st) {
+  switch (b.matter) {
+    case kDust: return go_constraints<O, kDust>(b, bg, cvals, cpart, st);
+    case kScalar: return go_constraints<O, kScalar>(b, bg, cvals, cpart, st);
+    case kStaticMatter: return go_constraints<O, kStaticMatter>(b, bg, cvals, cpart, st);
+    default: return go_constraints<O, kVacuum>(b, bg, cvals, cpart, st);
+  }
+}
+#endif
+
 #if !CG_AUX_UNIT
+template <int O, int M>
+cudaError_t go_group(const GroupBox* table, const GroupBg& gb, int stage, int grid, cudaStream_t st) {
+  constexpr size_t smem = stage_smem<O, M, kEvolve>();
+  static bool configured = false;
+  if (!configured) {
+    cudaError_t e = cudaFuncSetAttribute(stage_group_kernel<O, M>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (e != cudaSuccess) return e;
+    configured = true;
+  }
+  const int g = grid > 0 ? grid : gb.total;
+  stage_group_kernel<O, M><<<g, stage_block(), smem, st>>>(table, gb, stage);
+  return cudaGetLastError();
+}
+
+template <int O, int M>
+int ctas_per_sm() {
+  constexpr size_t smem = stage_smem<O, M, kEvolve>();
+  if (cudaFuncSetAttribute(stage_group_kernel<O, M>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) !=
+      cudaSuccess)
+    return 1;
+  int n = 0;
+  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, stage_group_kernel<O, M>, kThreads, smem) != cudaSuccess)
+    return 1;
+  return n > 0 ? n : 1;
+}
+
+template <int O>
+cudaError_t go_group_m(const GroupBox* table, const GroupBg& gb, int matter, int stage, int grid, cudaStream_t st) {
+  switch (matter) {
+    case kDust: return go_group<O, kDust>(table, gb, stage, grid, st);
+    case kScalar: return go_group<O, kScalar>(table, gb, stage, grid, st);
+    case kStaticMatter: return go_group<O, kStaticMatter>(table, gb, stage, grid, st);
+    default: return go_group<O, kVacuum>(table, gb, stage, grid, st);
+  }
+}
+template <int O>
+int ctas_m(int matter) {
+  switch (matter) {
+    case kDust: return ctas_per_sm<O, kDust>();
+    case kScalar: return ctas_per_sm<O, kScalar>();
+    case kStaticMatter: return ctas_per_sm<O, kStaticMatter>();
+    default: return ctas_per_sm<O, kVacuum>();
+  }
+}
+template <int O>
+bool encode_maps(BoxDev& b) {
+  using G = TileG<O>;
+  b.fmaps = 0;
+  if (!(tma_host::encode(&b.mapX, b.X, sizeof(double), b.nx, b.ny, b.nz, b.nfields, G::TZ, G::TY, G::TX) &&
+        tma_host::encode(&b.mapY, b.Y, sizeof(double), b.nx, b.ny, b.nz, b.nfields, G::TZ, G::TY, G::TX)))
+    return false;
+  if (b.FP0 && b.FP1) {  // dust: x, y, z boxes of the flux primitives
+    constexpr int R = O / 2;
+    const int box[3][3] = {{kBZ, kBY, kBX + 2 * R}, {kBZ, kBY + 2 * R, kBX}, {G::TZ, kBY, kBX}};
+    bool ok = true;
+    for (int a = 0; a < 3; ++a) {
+      ok = ok && tma_host::encode(&b.fmap0[a], b.FP0, sizeof(double), b.nx, b.ny, b.nz, P_N, box[a][0], box[a][1],
+                                  box[a][2]);
+      ok = ok && tma_host::encode(&b.fmap1[a], b.FP1, sizeof(double), b.nx, b.ny, b.nz, P_N, box[a][0], box[a][1],
+                                  box[a][2]);
+    }
+    b.fmaps = ok ? 1 : 0;
+  }
+  return true;
+}
+#endif  // !CG_AUX_UNIT
+}  // namespace
+
+template <>
+cudaError_t stage_of_order<CG_ORDER, kUnit>(const BoxDev& b, const StageBg& bg, int stage, cudaStream_t st) {
+  return go_stage_m<CG_ORDER>(b, bg, stage, st);
+}
+#if CG_REFERENCE_ORDER && !CG_SHIFT_UNIT
+template <>
+cudaError_t constraints_of_order<CG_ORDER, kUnit>(const BoxDev& b, const StageBg& bg, double* cvals, double* cpart,
+                                                  cudaStream_t st) {
+  return go_constraints_m<CG_ORDER>(b, bg, cvals, cpart, st);
+}
+#endif
+#if !CG_AUX_UNIT
+template <>
+cudaError_t group_of_order<CG_ORDER>(const GroupBox* table, const GroupBg& gb, int matter, int stage, int grid,
+                                     cudaStream_t st) {
+  return go_group_m<CG_ORDER>(table, gb, matter, stage, grid, st);
+}
+template <>
+int ctas_of_order<CG_ORDER>(int matter) {
+  return ctas_m<CG_ORDER>(matter);
+}
+template <>
+bool maps_of_order<CG_ORDER>(BoxDev& b) {
+  return encode_maps<CG_ORDER>(b);
+}
+#endif  // !CG_AUX_UNIT
+
+#else  // !CG_ORDER
+// ---- step initialisation and the choice of the order ---------------------------
 // BSSN::stepInit (bssn.cc:219-226) on the device: the first substep's input
 // is the normalised copy of _p (RK4Register::stepInit + set_DIFFgamma_Aij_norm);
 // for dust also the flux primitives of that input (Dust::stepInit ->
@@ -79,274 +318,62 @@ __global__ void __launch_bounds__(128) init_kernel(BoxGeom geo, Physics ph, Stag
   }
 }
 
-#endif  // !CG_AUX_UNIT
-
 namespace {
 dim3 block_dims() { return dim3(32, 4, 1); }
 dim3 grid_dims(const BoxDev& b) {
   return dim3((b.nz + 31) / 32, (b.ny + 3) / 4, b.nx);
 }
-dim3 stage_block() { return dim3(kBZ, kBY, kBX); }
-// bricks of the points a substep updates: x-slab boxes skip their ghost planes
-dim3 stage_grid(const BoxDev& b) {
-  return dim3((b.nz + kBZ - 1) / kBZ, (b.ny + kBY - 1) / kBY, (b.nx - 2 * b.xg + kBX - 1) / kBX);
-}
 
-template <int O, int M>
-cudaError_t go_stage(const BoxDev& b, const StageBg& bg, int stage, cudaStream_t st) {
-  StagePtrs P{};
-  P.kavg = b.kavg;
-  P.p = b.P;
-  P.f = b.F;
-  P.status = b.status;
-  switch (stage) {
-    case 1: P.in = b.X; P.prev = nullptr; P.out = b.Y; P.fp_in = b.FP0; P.fp_out = b.FP1; break;
-    case 2: P.in = b.Y; P.prev = b.X; P.out = b.X; P.fp_in = b.FP1; P.fp_out = b.FP0; break;
-    case 3: P.in = b.X; P.prev = b.Y; P.out = b.Y; P.fp_in = b.FP0; P.fp_out = b.FP1; break;
-    default: P.in = b.Y; P.prev = b.X; P.out = b.P; P.norm = b.X; P.fp_in = b.FP1; P.fp_out = b.FP0; break;
-  }
-  BoxGeom geo{b.nx, b.ny, b.nz, b.pts, b.xg / kBX};
-  const CUtensorMap& map = (stage == 1 || stage == 3) ? b.mapX : b.mapY;  // the substep's input
-  FluxMaps fm;
-  const CUtensorMap* fsrc = (stage == 1 || stage == 3) ? b.fmap0 : b.fmap1;
-  for (int a = 0; a < 3; ++a) fm.m[a] = fsrc[a];
-  constexpr bool Z = kZ4cUnit;
-  constexpr size_t smem = stage_smem<O, M, kEvolve, Z>();
-  if constexpr (kShiftUnit) {
-    // one instantiation per order and matter; the dissipation is switched at run time
-    static bool configured_shift = false;
-    if (!configured_shift) {
-      cudaError_t e = cudaFuncSetAttribute(stage_kernel<O, M, kEvolve, true, false, true>,
-                                           cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-      if (e != cudaSuccess) return e;
-      configured_shift = true;
-    }
-    stage_kernel<O, M, kEvolve, true, false, true><<<stage_grid(b), stage_block(), smem, st>>>(
-        geo, b.ph, bg, P, stage, map, b.tma, fm, b.fmaps);
-    return cudaGetLastError();
-  }
-  if constexpr (O == 2 || O == 8) {
-    if (b.ph.ko_coeff != 0.0) {  // Kreiss-Oliger dissipation: its own instantiation
-      static bool configured_ko = false;
-      if (!configured_ko) {
-        cudaError_t e = cudaFuncSetAttribute(stage_kernel<O, M, kEvolve, true, Z>,
-                                             cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-        if (e != cudaSuccess) return e;
-        configured_ko = true;
-      }
-      stage_kernel<O, M, kEvolve, true, Z><<<stage_grid(b), stage_block(), smem, st>>>(geo, b.ph, bg, P, stage, map,
-                                                                                       b.tma, fm, b.fmaps);
-      return cudaGetLastError();
-    }
-  }
-  static bool configured = false;  // per instantiation
-  if (!configured) {
-    cudaError_t e =
-        cudaFuncSetAttribute(stage_kernel<O, M, kEvolve, false, Z>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    if (e != cudaSuccess) return e;
-    configured = true;
-  }
-  stage_kernel<O, M, kEvolve, false, Z><<<stage_grid(b), stage_block(), smem, st>>>(geo, b.ph, bg, P, stage, map,
-                                                                                    b.tma, fm, b.fmaps);
-  return cudaGetLastError();
-}
-
-#if !CG_SHIFT_UNIT
-template <int O, int M>
-cudaError_t go_constraints(const BoxDev& b, const StageBg& bg, double* cvals, double* cpart, cudaStream_t st) {
-  StagePtrs P{};
-  P.in = b.X;
-  P.p = b.P;
-  P.fp_in = b.FP0;
-  P.status = b.status;
-  P.kavg = b.kavg;
-  P.cvals = cvals;
-  P.cpart = cpart;
-  BoxGeom geo{b.nx, b.ny, b.nz, b.pts, b.xg / kBX};
-  constexpr bool Z = kZ4cUnit;
-  constexpr size_t smem = stage_smem<O, M, kConstraints, Z>();
-  static bool configured = false;
-  if (!configured) {
-    cudaError_t e = cudaFuncSetAttribute(stage_kernel<O, M, kConstraints, false, Z>,
-                                         cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    if (e != cudaSuccess) return e;
-    configured = true;
-  }
-  FluxMaps fm{};
-  stage_kernel<O, M, kConstraints, false, Z><<<stage_grid(b), stage_block(), smem, st>>>(geo, b.ph, bg, P, 1, b.mapX,
-                                                                                         b.tma, fm, 0);
-  return cudaGetLastError();
-}
-
-template <int O>
-cudaError_t go_constraints_m(const BoxDev& b, const StageBg& bg, double* cvals, double* cpart, cudaStream_t st) {
-  switch (b.matter) {
-    case kDust: return go_constraints<O, kDust>(b, bg, cvals, cpart, st);
-    case kScalar: return go_constraints<O, kScalar>(b, bg, cvals, cpart, st);
-    case kStaticMatter: return go_constraints<O, kStaticMatter>(b, bg, cvals, cpart, st);
-    default: return go_constraints<O, kVacuum>(b, bg, cvals, cpart, st);
+// f(order tag) for the box's stencil order
+template <class F, class R>
+R by_order(int order, F f, R other) {
+  switch (order) {
+    case 2: return f(std::integral_constant<int, 2>());
+    case 4: return f(std::integral_constant<int, 4>());
+    case 6: return f(std::integral_constant<int, 6>());
+    case 8: return f(std::integral_constant<int, 8>());
+    default: return other;
   }
 }
-#endif  // !CG_SHIFT_UNIT
-
-#if !CG_AUX_UNIT
-template <int O, int M>
-cudaError_t go_group(const GroupBox* table, const GroupBg& gb, int stage, int grid, cudaStream_t st) {
-  constexpr size_t smem = stage_smem<O, M, kEvolve>();
-  static bool configured = false;
-  if (!configured) {
-    cudaError_t e = cudaFuncSetAttribute(stage_group_kernel<O, M>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    if (e != cudaSuccess) return e;
-    configured = true;
-  }
-  const int g = grid > 0 ? grid : gb.total;
-  stage_group_kernel<O, M><<<g, stage_block(), smem, st>>>(table, gb, stage);
-  return cudaGetLastError();
-}
-
-template <int O, int M>
-int ctas_per_sm() {
-  constexpr size_t smem = stage_smem<O, M, kEvolve>();
-  if (cudaFuncSetAttribute(stage_group_kernel<O, M>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) !=
-      cudaSuccess)
-    return 1;
-  int n = 0;
-  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, stage_group_kernel<O, M>, kThreads, smem) != cudaSuccess)
-    return 1;
-  return n > 0 ? n : 1;
-}
-
-template <int O>
-cudaError_t go_group_m(const GroupBox* table, const GroupBg& gb, int matter, int stage, int grid, cudaStream_t st) {
-  switch (matter) {
-    case kDust: return go_group<O, kDust>(table, gb, stage, grid, st);
-    case kScalar: return go_group<O, kScalar>(table, gb, stage, grid, st);
-    case kStaticMatter: return go_group<O, kStaticMatter>(table, gb, stage, grid, st);
-    default: return go_group<O, kVacuum>(table, gb, stage, grid, st);
-  }
-}
-template <int O>
-int ctas_m(int matter) {
-  switch (matter) {
-    case kDust: return ctas_per_sm<O, kDust>();
-    case kScalar: return ctas_per_sm<O, kScalar>();
-    case kStaticMatter: return ctas_per_sm<O, kStaticMatter>();
-    default: return ctas_per_sm<O, kVacuum>();
-  }
-}
-
-#endif  // !CG_AUX_UNIT
-
-template <int O>
-cudaError_t go_stage_m(const BoxDev& b, const StageBg& bg, int stage, cudaStream_t st) {
-  switch (b.matter) {
-    case kDust: return go_stage<O, kDust>(b, bg, stage, st);
-    case kScalar: return go_stage<O, kScalar>(b, bg, stage, st);
-#if !CG_SHIFT_UNIT  // static matter has no shift (cg_create rejects it)
-    case kStaticMatter: return go_stage<O, kStaticMatter>(b, bg, stage, st);
-#endif
-    default: return go_stage<O, kVacuum>(b, bg, stage, st);
-  }
-}
-#if !CG_AUX_UNIT
-template <int O>
-bool encode_maps(BoxDev& b) {
-  using G = TileG<O>;
-  b.fmaps = 0;
-  if (!(tma_host::encode(&b.mapX, b.X, sizeof(double), b.nx, b.ny, b.nz, b.nfields, G::TZ, G::TY, G::TX) &&
-        tma_host::encode(&b.mapY, b.Y, sizeof(double), b.nx, b.ny, b.nz, b.nfields, G::TZ, G::TY, G::TX)))
-    return false;
-  if (b.FP0 && b.FP1) {  // dust: x, y, z boxes of the flux primitives
-    constexpr int R = O / 2;
-    const int box[3][3] = {{kBZ, kBY, kBX + 2 * R}, {kBZ, kBY + 2 * R, kBX}, {G::TZ, kBY, kBX}};
-    bool ok = true;
-    for (int a = 0; a < 3; ++a) {
-      ok = ok && tma_host::encode(&b.fmap0[a], b.FP0, sizeof(double), b.nx, b.ny, b.nz, P_N, box[a][0], box[a][1],
-                                  box[a][2]);
-      ok = ok && tma_host::encode(&b.fmap1[a], b.FP1, sizeof(double), b.nx, b.ny, b.nz, P_N, box[a][0], box[a][1],
-                                  box[a][2]);
-    }
-    b.fmaps = ok ? 1 : 0;
-  }
-  return true;
-}
-#endif  // !CG_AUX_UNIT
 }  // namespace
 
-#if !CG_AUX_UNIT
 void make_tile_maps(BoxDev& b) {
-  bool ok = false;
-  switch (b.order) {
-    case 2: ok = encode_maps<2>(b); break;
-    case 4: ok = encode_maps<4>(b); break;
-    case 6: ok = encode_maps<6>(b); break;
-    case 8: ok = encode_maps<8>(b); break;
-    default: break;
-  }
-  b.maps = b.tma = ok ? 1 : 0;
+  b.maps = b.tma = by_order(b.order, [&](auto o) { return maps_of_order<o.value>(b); }, false) ? 1 : 0;
 }
 
-#endif  // !CG_AUX_UNIT
-
-#if !CG_AUX_UNIT && !CG_REFERENCE_ORDER
-// the shift is built into the parity build only; cg_create accepts it with CG_PREC_FP64 alone
-cudaError_t launch_stage_shift(const BoxDev&, const StageBg&, int, cudaStream_t) { return cudaErrorNotSupported; }
-#endif
-
-#if CG_Z4C_UNIT
-cudaError_t launch_stage_z4c(const BoxDev& b, const StageBg& bg, int stage, cudaStream_t st) {
-#elif CG_SHIFT_UNIT
-cudaError_t launch_stage_shift(const BoxDev& b, const StageBg& bg, int stage, cudaStream_t st) {
-#else
 cudaError_t launch_stage(const BoxDev& b, const StageBg& bg, int stage, cudaStream_t st) {
-  if (b.z4c) return launch_stage_z4c(b, bg, stage, st);
-  if (b.shift) return launch_stage_shift(b, bg, stage, st);
+  return by_order(
+      b.order,
+      [&](auto o) {
+        if (b.z4c) return stage_of_order<o.value, 1>(b, bg, stage, st);
+#if CG_REFERENCE_ORDER  // the shift is built into the parity build only; cg_create accepts it with CG_PREC_FP64 alone
+        if (b.shift) return stage_of_order<o.value, 2>(b, bg, stage, st);
 #endif
-  switch (b.order) {
-    case 2: return go_stage_m<2>(b, bg, stage, st);
-    case 4: return go_stage_m<4>(b, bg, stage, st);
-    case 6: return go_stage_m<6>(b, bg, stage, st);
-    case 8: return go_stage_m<8>(b, bg, stage, st);
-    default: return cudaErrorInvalidValue;
-  }
+        return stage_of_order<o.value, 0>(b, bg, stage, st);
+      },
+      cudaErrorInvalidValue);
 }
 
-#if !CG_SHIFT_UNIT  // shift boxes take the constraint statistics of the plain kernels
-#if CG_Z4C_UNIT
-cudaError_t launch_constraints_z4c(const BoxDev& b, const StageBg& bg, double* cvals, double* cpart, cudaStream_t st) {
-#else
+#if CG_REFERENCE_ORDER
 cudaError_t launch_constraints(const BoxDev& b, const StageBg& bg, double* cvals, double* cpart, cudaStream_t st) {
-  if (b.z4c) return launch_constraints_z4c(b, bg, cvals, cpart, st);
-#endif
-  switch (b.order) {
-    case 2: return go_constraints_m<2>(b, bg, cvals, cpart, st);
-    case 4: return go_constraints_m<4>(b, bg, cvals, cpart, st);
-    case 6: return go_constraints_m<6>(b, bg, cvals, cpart, st);
-    case 8: return go_constraints_m<8>(b, bg, cvals, cpart, st);
-    default: return cudaErrorInvalidValue;
-  }
+  return by_order(
+      b.order,
+      [&](auto o) {
+        return b.z4c ? constraints_of_order<o.value, 1>(b, bg, cvals, cpart, st)
+                     : constraints_of_order<o.value, 0>(b, bg, cvals, cpart, st);
+      },
+      cudaErrorInvalidValue);
 }
-#endif  // !CG_SHIFT_UNIT
+#endif
 
-#if !CG_AUX_UNIT
 cudaError_t launch_group(const GroupBox* table, const GroupBg& gb, int order, int matter, int stage, int grid,
                          cudaStream_t st) {
-  switch (order) {
-    case 2: return go_group_m<2>(table, gb, matter, stage, grid, st);
-    case 4: return go_group_m<4>(table, gb, matter, stage, grid, st);
-    case 6: return go_group_m<6>(table, gb, matter, stage, grid, st);
-    case 8: return go_group_m<8>(table, gb, matter, stage, grid, st);
-    default: return cudaErrorInvalidValue;
-  }
+  return by_order(
+      order, [&](auto o) { return group_of_order<o.value>(table, gb, matter, stage, grid, st); }, cudaErrorInvalidValue);
 }
 
 int group_ctas_per_sm(int order, int matter) {
-  switch (order) {
-    case 2: return ctas_m<2>(matter);
-    case 4: return ctas_m<4>(matter);
-    case 6: return ctas_m<6>(matter);
-    default: return ctas_m<8>(matter);
-  }
+  return by_order(order, [&](auto o) { return ctas_of_order<o.value>(matter); }, 1);
 }
 
 int constraint_blocks(const BoxDev& b) {
@@ -372,7 +399,7 @@ cudaError_t launch_init(const BoxDev& b, const StageBg& bg, cudaStream_t st) {
   return cudaGetLastError();
 }
 
-#endif  // !CG_AUX_UNIT
+#endif  // CG_ORDER
 
 }  // namespace CG_VARIANT_NS
 }  // namespace cg
