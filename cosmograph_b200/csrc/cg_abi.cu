@@ -895,6 +895,7 @@ int cg_create(const cg_box_desc* boxes, int nboxes, cg_ctx** out) {
     ph.normalize = d.normalize_metric;
     ph.dx = d.dx;
     ph.inv_dx = 1.0 / d.dx;
+    ph.inv_dx_lo = std::fma(-d.dx, ph.inv_dx, 1.0) / d.dx;
     ph.dx_pow2 = is_pow2(d.dx) ? 1 : 0;
     ph.dt = d.dt;
     ph.lambda = d.lambda;

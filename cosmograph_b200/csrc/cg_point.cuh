@@ -66,103 +66,80 @@ __device__ __forceinline__ int wrap(int v, int n) {
   return v >= n ? v - n : v;
 }
 
-// Periodic neighbourhood of one grid point; linear index within one field.
-struct Site {
-  int i, j, k, nx, ny, nz;
-  __device__ __forceinline__ int at(int di, int dj, int dk) const {
-    return (wrap(i + di, nx) * ny + wrap(j + dj, ny)) * nz + wrap(k + dk, nz);
+// Division by a divisor known in advance: x / d rounded as IEEE division
+// rounds it, from hi = RN(1/d) and lo = 1/d - hi (Brisebarre, Muller and
+// Raina, IEEE Trans. Computers 53(8), 2004): q = x hi + x lo is within an ulp
+// of x / d, the remainder x - q d is exact in one fma, and Markstein's theorem
+// (IBM J. Res. Dev. 34(1), 1990) makes q + remainder hi the correctly rounded
+// quotient.  Holds while nothing under- or overflows: |d| in [2^-100, 2^100]
+// and x = 0 or |x| in [2^-800, 2^800], which DivRange checks for a batch of
+// numerators at a time (a quotient of zero may come out as the other zero).
+// Four dependent operations against the longer chain and the branch of a
+// general division, whose blocks also kept independent quotients apart.
+struct Divisor {
+  double d, hi, lo;
+  __device__ __forceinline__ double operator()(double x) const {
+    const double q = __fma_rn(x, hi, __dmul_rn(x, lo));
+    return __fma_rn(__fma_rn(-d, q, x), hi, q);
   }
-  __device__ __forceinline__ int ax(int a, int n) const {
-    return at(a == 0 ? n : 0, a == 1 ? n : 0, a == 2 ? n : 0);
+};
+__device__ __forceinline__ Divisor divisor(double d) {
+  const double hi = 1.0 / d;
+  return Divisor{d, hi, __dmul_rn(__fma_rn(-d, hi, 1.0), hi)};
+}
+struct DivRange {
+  // the exponent fields (sign dropped) of the largest numerator and, with
+  // zero mapped to the top, of the smallest
+  unsigned top = 0, low = 0xffffffffu;
+  __device__ __forceinline__ void numerator(double x) {
+    const unsigned h = (unsigned)__double2hiint(x) << 1;
+    top = max(top, h);
+    low = min(low, (h | min((unsigned)__double2loint(x), 1u)) - 1u);
   }
-  __device__ __forceinline__ int pl(int a, int n, int b, int m) const {
-    int o[3] = {0, 0, 0};
-    o[a] += n;
-    o[b] += m;
-    return at(o[0], o[1], o[2]);
+  __device__ __forceinline__ bool ok() const { return top < (1823u << 21) && low >= (223u << 21); }
+  // a divisor in [2^-100, 2^100]
+  __device__ __forceinline__ static bool divisor_ok(double d) {
+    return (((unsigned)__double2hiint(d) << 1) >> 21) - 923u <= 200u;
   }
 };
 
-template <typename T>
-__device__ __forceinline__ T ld(const T* __restrict__ p, int idx) {
-  return __ldg(p + idx);
+// sums[q] / dx, the first N1 once and the rest twice, bit-identical to the
+// reference's divisions: a multiply when dx is a power of two, where both
+// round identically.  One choice for a whole batch, so that the sums before
+// it are one block of independent chains.
+template <int N, int N1>
+__device__ __forceinline__ void div_dx(double (&sums)[N], const Physics& ph) {
+  if (ph.dx_pow2) {
+#pragma unroll
+    for (int q = 0; q < N; ++q) {
+      sums[q] = sums[q] * ph.inv_dx;
+      if (q >= N1) sums[q] = sums[q] * ph.inv_dx;
+    }
+    return;
+  }
+  DivRange rg;
+#pragma unroll
+  for (int q = 0; q < N; ++q) rg.numerator(sums[q]);
+  if (rg.ok() && DivRange::divisor_ok(ph.dx)) {
+    const Divisor by{ph.dx, ph.inv_dx, ph.inv_dx_lo};
+#pragma unroll
+    for (int q = 0; q < N; ++q) {
+      sums[q] = by(sums[q]);
+      if (q >= N1) sums[q] = by(sums[q]);
+    }
+    return;
+  }
+#pragma unroll
+  for (int q = 0; q < N; ++q) {
+    sums[q] = sums[q] / ph.dx;
+    if (q >= N1) sums[q] = sums[q] / ph.dx;
+  }
 }
 
 // x/dx, bit-identical to the reference's division (a multiply when dx is a
 // power of two, where both round identically).
 __device__ __forceinline__ double divdx(double x, const Physics& ph) {
   return ph.dx_pow2 ? x * ph.inv_dx : x / ph.dx;
-}
-
-// First derivative along axis a: utils/math.h:74-100, 231-263, 412-450, 554-586.
-template <int O>
-__device__ __forceinline__ double der1(const double* __restrict__ f, const Site& s, int a,
-                                       const Physics& ph) {
-  auto V = [&](int n) { return ld(f, s.ax(a, n)); };
-  double t;
-  if (O == 2) {
-    t = (-1.0 / 2.0 * V(-1) + 1.0 / 2.0 * V(1));
-  } else if (O == 4) {
-    t = (+1.0 / 12.0 * V(-2) - 2.0 / 3.0 * V(-1) + 2.0 / 3.0 * V(1) - 1.0 / 12.0 * V(2));
-  } else if (O == 6) {
-    t = (-1.0 / 60.0 * V(-3) + 3.0 / 20.0 * V(-2) - 3.0 / 4.0 * V(-1) + 3.0 / 4.0 * V(1) -
-         3.0 / 20.0 * V(2) + 1.0 / 60.0 * V(3));
-  } else {
-    t = ((1.0 / 280.0 * V(-4) - 1.0 / 280.0 * V(4)) - (4.0 / 105.0 * V(-3) - 4.0 / 105.0 * V(3)) +
-         (1.0 / 5.0 * V(-2) - 1.0 / 5.0 * V(2)) - (4.0 / 5.0 * V(-1) - 4.0 / 5.0 * V(1)));
-  }
-  return divdx(t, ph);
-}
-
-// Second derivative along axis a: utils/math.h:857-885, 958-993, 995-1036, 1038-1085.
-template <int O>
-__device__ __forceinline__ double der2(const double* __restrict__ f, const Site& s, int a,
-                                       const Physics& ph) {
-  auto V = [&](int n) { return ld(f, s.ax(a, n)); };
-  double t;
-  if (O == 2) {
-    t = (V(-1) - 2.0 * V(0) + V(1));
-  } else if (O == 4) {
-    t = (-1.0 / 12.0 * V(-2) + 4.0 / 3.0 * V(-1) - 5.0 / 2.0 * V(0) + 4.0 / 3.0 * V(1) -
-         1.0 / 12.0 * V(2));
-  } else if (O == 6) {
-    t = (1.0 / 90.0 * V(-3) - 3.0 / 20.0 * V(-2) + 3.0 / 2.0 * V(-1) - 49.0 / 18.0 * V(0) +
-         3.0 / 2.0 * V(1) - 3.0 / 20.0 * V(2) + 1.0 / 90.0 * V(3));
-  } else {
-    t = (-1.0 / 560.0 * V(-4) + 8.0 / 315.0 * V(-3) - 1.0 / 5.0 * V(-2) + 8.0 / 5.0 * V(-1) -
-         205.0 / 72.0 * V(0) + 8.0 / 5.0 * V(1) - 1.0 / 5.0 * V(2) + 8.0 / 315.0 * V(3) -
-         1.0 / 560.0 * V(4));
-  }
-  return divdx(divdx(t, ph), ph);
-}
-
-// Mixed second derivative on axes a < b: utils/math.h:676-855.
-template <int O>
-__device__ __forceinline__ double derm(const double* __restrict__ f, const Site& s, int a, int b,
-                                       const Physics& ph) {
-  auto P = [&](int n) {
-    return -ld(f, s.pl(a, n, b, -n)) + ld(f, s.pl(a, n, b, n)) + ld(f, s.pl(a, -n, b, -n)) -
-           ld(f, s.pl(a, -n, b, n));
-  };
-  double t;
-  if (O == 2) {
-    t = P(1) / 4.0;
-  } else if (O == 4) {
-    t = (P(1) - 1.0 / 16.0 * P(2)) / 3.0;
-  } else if (O == 6) {
-    t = (135.0 * P(1) - 27.0 / 2.0 * P(2) + P(3)) / 360.0;
-  } else {
-    t = (2.0 / 5.0 * P(1) - 1.0 / 20.0 * P(2) + 2.0 / 315.0 * P(3) - 1.0 / 2240.0 * P(4));
-  }
-  return divdx(divdx(t, ph), ph);
-}
-
-// utils/math.h:1319-1330
-template <int O>
-__device__ __forceinline__ double der2ab(const double* __restrict__ f, const Site& s, int a, int b,
-                                        const Physics& ph) {
-  if (a == b) return der2<O>(f, s, a, ph);
-  return a < b ? derm<O>(f, s, a, b, ph) : derm<O>(f, s, b, a, ph);
 }
 
 // Inverse conformal metric assuming unit determinant, bssn.cc:447-455.

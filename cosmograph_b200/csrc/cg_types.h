@@ -39,6 +39,7 @@ struct Physics {
   int matter, lapse, potential, normalize;
   double dx, inv_dx, dt;
   int dx_pow2;            // dx is a power of two: x/dx == x*inv_dx exactly
+  double inv_dx_lo;       // 1/dx - inv_dx (Divisor, cg_point.cuh)
   double lambda;          // rho_Lambda
   double a_adj_amp, k_damping_amp, gd_c, dw_mu_l, dw_p;
   double pot_const, pot_mass;
