@@ -96,7 +96,9 @@ struct DivRange {
     top = max(top, h);
     low = min(low, (h | min((unsigned)__double2loint(x), 1u)) - 1u);
   }
-  __device__ __forceinline__ bool ok() const { return top < (1823u << 21) && low >= (223u << 21); }
+  // every numerator zero or in [2^-e, 2^e]
+  __device__ __forceinline__ bool within(unsigned e) const { return top < ((1023u + e) << 21) && low >= ((1023u - e) << 21); }
+  __device__ __forceinline__ bool ok() const { return within(800); }
   // a divisor in [2^-100, 2^100]
   __device__ __forceinline__ static bool divisor_ok(double d) {
     return (((unsigned)__double2hiint(d) << 1) >> 21) - 923u <= 200u;
@@ -198,15 +200,33 @@ __device__ __forceinline__ DustPrim dust_prim(const double gi[6], double em4phi,
 // (W, det g, g_ij of the previous populate) and the current D, S_i.
 __device__ __forceinline__ void dust_sources(double W, double detg, const double gphys[6], double D,
                                              const double S[3], double lambda, double q[Q_N]) {
-  q[Q_R] = W * D / detg;
-  const double Sd = D / detg * (W * W - 1.0) / W;
-  q[Q_S] = Sd;
-  for (int m = 0; m < 3; ++m) q[Q_S1 + m] = S[m] / detg;
+  // 24 quotients by W, D and detg: their reciprocals once (Divisor), unless
+  // something leaves its range
+  const double ss[6] = {S[0] * S[0], S[0] * S[1], S[0] * S[2], S[1] * S[1], S[1] * S[2], S[2] * S[2]};
+  DivRange rg;
+  rg.numerator(W * D);
 #pragma unroll
-  for (int I = 0; I < 3; ++I)
+  for (int m = 0; m < 3; ++m) rg.numerator(S[m]);
 #pragma unroll
-    for (int J = I; J < 3; ++J)
-      q[Q_STF11 + sym(I, J)] = S[I] * S[J] / W / D / detg - 1.0 / 3.0 * gphys[sym(I, J)] * Sd;
+  for (int m = 0; m < 6; ++m) rg.numerator(ss[m]);
+  const double w2 = W * W - 1.0;
+  if (rg.within(256) && DivRange::divisor_ok(W) && DivRange::divisor_ok(D) && DivRange::divisor_ok(detg)) {
+    const Divisor byW = divisor(W), byD = divisor(D), byV = divisor(detg);
+    q[Q_R] = byV(W * D);
+    const double Sd = byW(byV(D) * w2);
+    q[Q_S] = Sd;
+#pragma unroll
+    for (int m = 0; m < 3; ++m) q[Q_S1 + m] = byV(S[m]);
+#pragma unroll
+    for (int m = 0; m < 6; ++m) q[Q_STF11 + m] = byV(byD(byW(ss[m]))) - 1.0 / 3.0 * gphys[m] * Sd;
+  } else {
+    q[Q_R] = W * D / detg;
+    const double Sd = D / detg * w2 / W;
+    q[Q_S] = Sd;
+    for (int m = 0; m < 3; ++m) q[Q_S1 + m] = S[m] / detg;
+#pragma unroll
+    for (int m = 0; m < 6; ++m) q[Q_STF11 + m] = ss[m] / W / D / detg - 1.0 / 3.0 * gphys[m] * Sd;
+  }
   q[Q_R] += lambda;
   q[Q_S] += -3.0 * lambda;
 }

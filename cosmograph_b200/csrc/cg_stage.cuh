@@ -164,6 +164,9 @@ __device__ __forceinline__ StagePtrs group_ptrs(const GroupBox& b, int stage) {
 
 namespace CG_VARIANT_NS {
 
+// 1/6 - RN(1/6); twice that for 1/3 (Divisor)
+constexpr double kSixthLo = 0x1.5555555555555p-57;
+
 // Stencil taps of one point.  WRAP=false: the brick lies at least r points
 // from every face, taps are plain offsets.  WRAP=true: periodic wrap.
 template <bool WRAP>
@@ -472,10 +475,7 @@ __device__ __forceinline__ void field_derivatives(int it, const tile::Taps<TileG
       // bssn_macros.h:248-249, summed over (k,l) in the reference's order).
       // The nine sums first and their divisions in one batch: independent
       // chains in one block, where a choice of the division per sum kept
-      // them apart.  What bounds the kernel is the latency of dependent FP64
-      // operations, so this took the dust step from 85.3 to 73.8 ms at 256^3
-      // (order 8) and, where dx is no power of two, from 43.9 to 34.6 ms at
-      // 192^3.
+      // them apart.
       const int q = it - PF::NA;
       double s[9] = {s1<O>(t, 0), s1<O>(t, 1), s1<O>(t, 2), s2<O>(t, 0),    s2<O>(t, 1),
                      s2<O>(t, 2), sm<O>(t, 0, 1), sm<O>(t, 0, 2), sm<O>(t, 1, 2)};
@@ -842,33 +842,47 @@ __device__ __forceinline__ void stage_body(const BoxGeom& geo, const Physics& ph
     }
   }
   const double divb = (db[0][0] + db[1][1]) + db[2][2];
-  // every e^x this point's substep takes, in one batch: of phi and, for dust
-  // after the first substep, of the previous substep's phi (the lagged
-  // sources); static matter takes e^{-6 phi} in the sixth place
+  // The Hamiltonian constraint enters the right-hand sides through a_adj_amp
+  // and k_damping_amp only (and through Z4c's theta by its own expression):
+  // with both zero its terms are zero times H, and neither H nor its e^{5 phi}
+  // and e^{-5 phi} are formed.
+  const bool need_H = MODE == kConstraints || ph.a_adj_amp != 0.0 || ph.k_damping_amp != 0.0;
+  // every e^x this point's substep takes, in one batch: -4 phi, 4 phi; 6 phi
+  // (dust, and the momentum constraint); for dust after the first substep the
+  // same three of the previous substep's phi (the lagged sources); -6 phi
+  // (static matter); last 5 phi and -5 phi, taken with need_H
   double phip = phi;
   if (MATTER == kDust && stage > 1) phip = __ldcs(&P.prev[(size_t)F_PHI * N + c]) + bg.phi_FRW_prev;
-  // (without dust the previous substep's phi is not needed: five values, six
-  // with static matter)
   // The parity build evaluates the batch through this thread's slots of the
   // Christoffel symbols (free until they are formed): arguments in S_G,
   // results in S_G + NX, the fast evaluation in a rolled loop (one copy of its
   // code, which stays in the instruction cache), the accurate phase for the
   // undecided ones after it; the same correctly rounded values as xexp_n.
-  constexpr int NX = MATTER == kDust ? 8 : (MATTER == kStaticMatter ? 6 : 5);
+  constexpr int X6 = MATTER == kDust || MODE == kConstraints ? 1 : 0;     // 6 phi
+  constexpr int XM = MATTER == kDust ? 3 : (MATTER == kStaticMatter ? 1 : 0);  // the lagged three, or -6 phi
+  constexpr int X5 = 2 + X6 + XM, NX = X5 + 2;
   static_assert(2 * NX <= 18, "the batch fits the Christoffel slots");
-  double ex[8];
+  double ex[NX];
   {
     double xa[NX];
-#pragma unroll
-    for (int q = 0; q < NX; ++q)
-      xa[q] = q < 5 ? (q == 0 ? -4.0 : q == 1 ? 4.0 : q == 2 ? 6.0 : q == 3 ? 5.0 : -5.0) * phi
-                    : (MATTER == kStaticMatter ? -6.0 * phi : (q == 5 ? -4.0 : q == 6 ? 4.0 : 6.0) * phip);
+    xa[0] = -4.0 * phi;
+    xa[1] = 4.0 * phi;
+    if constexpr (X6 != 0) xa[2] = 6.0 * phi;
+    if constexpr (MATTER == kDust) {
+      xa[2 + X6] = -4.0 * phip;
+      xa[3 + X6] = 4.0 * phip;
+      xa[4 + X6] = 6.0 * phip;
+    }
+    if constexpr (MATTER == kStaticMatter) xa[2 + X6] = -6.0 * phi;
+    xa[X5] = 5.0 * phi;
+    xa[X5 + 1] = -5.0 * phi;
+    const int nx = need_H ? NX : X5;
     if constexpr (kReferenceOrder) {
 #pragma unroll
       for (int q = 0; q < NX; ++q) S(S_G + q) = xa[q];
       unsigned bad = 0;
 #pragma unroll 1
-      for (int q = 0; q < NX; ++q) {
+      for (int q = 0; q < nx; ++q) {
         double y;
         if (!crm::exp_fast(S(S_G + q), y)) bad |= 1u << q;
         S(S_G + NX + q) = y;
@@ -882,19 +896,17 @@ __device__ __forceinline__ void stage_body(const BoxGeom& geo, const Physics& ph
 #pragma unroll
       for (int q = 0; q < NX; ++q) ex[q] = S(S_G + NX + q);
     } else {
-      double ey[NX];
-      xexp_n<NX>(xa, ey);
 #pragma unroll
-      for (int q = 0; q < NX; ++q) ex[q] = ey[q];
+      for (int q = 0; q < X5; ++q) ex[q] = xexp(xa[q]);
+#pragma unroll
+      for (int q = X5; q < NX; ++q) ex[q] = need_H ? xexp(xa[q]) : 0.0;
     }
   }
-  if constexpr (NX < 8) {  // without dust the previous substep's phi is this one's
-    if constexpr (NX == 5) ex[5] = ex[0];
-    ex[6] = ex[1];
-    ex[7] = ex[2];
-  }
-  const double em4phi = ex[0], e4phi = ex[1], e6phi = ex[2], e5phi = ex[3], em5phi = ex[4];
-  const double em4phip = ex[5], e4phip = ex[6], e6phip = ex[7];
+  const double em4phi = ex[0], e4phi = ex[1];
+  const double e6phi = X6 ? ex[2] : 0.0, e5phi = ex[X5], em5phi = ex[X5 + 1];
+  // the lagged three (dust; the same state's at the first substep)
+  const double em4phip = ex[MATTER == kDust ? 3 : 0], e4phip = ex[MATTER == kDust ? 4 : 0],
+               e6phip = ex[MATTER == kDust ? 5 : 0];
 
   // -- sources and matter centre quantities --
   double rhs_m[5] = {0, 0, 0, 0, 0};
@@ -1016,7 +1028,7 @@ __device__ __forceinline__ void stage_body(const BoxGeom& geo, const Physics& ph
     for (int m = 0; m < Q_N; ++m) S(S_SRC + m) = 0.0;
     const double phid = C(F_PHI);
     double r = 0.0;
-    r += ex[5] * C(F_DIFFD) + bg.rho_FRW * xexpm1(-6.0 * phid);
+    r += ex[2 + X6] * C(F_DIFFD) + bg.rho_FRW * xexpm1(-6.0 * phid);
     r += ph.lambda;
     S(S_SRC + Q_R) = r;
     S(S_SRC + Q_S) = 0.0 + -3.0 * ph.lambda;
@@ -1026,40 +1038,33 @@ __device__ __forceinline__ void stage_body(const BoxGeom& geo, const Physics& ph
   }
 
   // -- Christoffels (bssn.cc:577-590, bssn_macros.h:221-229) --
-  // Gamma^I_q go to their own slots; the lowered Gamma_{I q} then replace
-  // d_I g_q, which nothing reads afterwards.
-  // the pair (J, K) in a rolled loop (slot addresses at run time, one copy of
-  // the code), the three brackets shared by the three I
-#pragma unroll 1
-  for (int q = 0; q < 6; ++q) {
-    const int J = q < 3 ? 0 : (q < 5 ? 1 : 2), Kx = q < 3 ? q : (q < 5 ? q - 2 : 2);  // sym(J, Kx) = q
-    auto dg = [&](int d, int qq) { return S(S_DG + 6 * d + qq); };
-    const double b0 = dg(J, sym(Kx, 0)) + dg(Kx, sym(J, 0)) - dg(0, q);
-    const double b1 = dg(J, sym(Kx, 1)) + dg(Kx, sym(J, 1)) - dg(1, q);
-    const double b2 = dg(J, sym(Kx, 2)) + dg(Kx, sym(J, 2)) - dg(2, q);
-#pragma unroll
-    for (int I = 0; I < 3; ++I) {
-      double u = gi[sym(I, 0)] * (b0);
-      u = u + gi[sym(I, 1)] * (b1);
-      u = u + gi[sym(I, 2)] * (b2);
-      S(S_G + 6 * I + q) = 0.5 * (u);
-    }
-  }
+  // The 18 d_I g_q are read once; the brackets d_J g_KI + d_K g_JI - d_I g_JK
+  // give the lowered symbols (half of each, which replace d_I g_q in their
+  // slots: nothing reads those afterwards) and, contracted with g^{IL}, the
+  // raised ones.
   {
-    double GLv[3][6];
+    double dg[18];
 #pragma unroll
-    for (int I = 0; I < 3; ++I)
+    for (int q = 0; q < 18; ++q) dg[q] = S(S_DG + q);
 #pragma unroll
-      for (int J = 0; J < 3; ++J)
+    for (int J = 0; J < 3; ++J)
 #pragma unroll
-        for (int Kx = J; Kx < 3; ++Kx) {
-          auto dg = [&](int d, int qq) { return S(S_DG + 6 * d + qq); };
-          GLv[I][sym(J, Kx)] = 0.5 * (dg(J, sym(Kx, I)) + dg(Kx, sym(J, I)) - dg(I, sym(J, Kx)));
+      for (int Kx = J; Kx < 3; ++Kx) {
+        const int q = sym(J, Kx);
+        double b[3];
+#pragma unroll
+        for (int I = 0; I < 3; ++I) {
+          b[I] = dg[6 * J + sym(Kx, I)] + dg[6 * Kx + sym(J, I)] - dg[6 * I + q];
+          S(S_DG + 6 * I + q) = 0.5 * b[I];
         }
 #pragma unroll
-    for (int I = 0; I < 3; ++I)
-#pragma unroll
-      for (int qq = 0; qq < 6; ++qq) S(S_DG + 6 * I + qq) = GLv[I][qq];
+        for (int I = 0; I < 3; ++I) {
+          double u = gi[sym(I, 0)] * b[0];
+          u = u + gi[sym(I, 1)] * b[1];
+          u = u + gi[sym(I, 2)] * b[2];
+          S(S_G + 6 * I + q) = 0.5 * (u);
+        }
+      }
   }
   auto G = [&](int I, int qq) { return S(S_G + 6 * I + qq); };
   auto GL = [&](int I, int qq) { return S(S_DG + 6 * I + qq); };
@@ -1200,7 +1205,7 @@ __device__ __forceinline__ void stage_body(const BoxGeom& geo, const Physics& ph
   const double AijAij = Ac[0] * A[0] + Ac[3] * A[3] + Ac[5] * A[5] + 2.0 * (Ac[1] * A[1] + Ac[2] * A[2] + Ac[4] * A[4]);
   const double r = S(S_SRC + Q_R) + bg.rho_FRW;
   // Hamiltonian constraint, bssn.cc:1073-1084 (theta = 0)
-  const double H = -e5phi / 8.0 * (ricci + 2.0 / 3.0 * ((K + 2.0 * theta) * (K + 2.0 * theta)) - AijAij - 16.0 * kPi * r);
+  const double H = need_H ? -e5phi / 8.0 * (ricci + 2.0 / 3.0 * ((K + 2.0 * theta) * (K + 2.0 * theta)) - AijAij - 16.0 * kPi * r) : 0.0;
 
   if constexpr (MODE == kConstraints) {
     // BSSN::setConstraintCalcs per point (bssn.cc:983-1006)
@@ -1525,12 +1530,15 @@ __device__ __forceinline__ void stage_body(const BoxGeom& geo, const Physics& ph
   // rolled loop (one copy of the code) with the next field's registers
   // loaded while this one is updated; the substep's divisors chosen once:
   // f = f + dt cv / 6 (substep 1, from f = 0), / 3 (2, 3); a = p + dt cv / 2
-  // (1, 2), / 1 (3); p = f + (dt cv / 6 + p) (4).  IEEE division rounds the
-  // same for a divisor held in a register, and 0 + x = x, so the values are
-  // those of the four separate forms.  The new values replace the
+  // (1, 2), / 1 (3); p = f + (dt cv / 6 + p) (4).  0 + x = x, so the values
+  // are those of the four separate forms.  The new values replace the
   // right-hand sides in the slots.
   {
-    const double fdiv = stage == 1 ? 6.0 : 3.0, odiv = stage == 3 ? 1.0 : 2.0;
+    // the quotient by 6 (substeps 1 and 4) or 3 through the divisor's
+    // reciprocal; the half (substeps 1, 2) is exact as a product
+    const bool by6 = stage == 1 || stage == 4;
+    const Divisor by{by6 ? 6.0 : 3.0, by6 ? 1.0 / 6.0 : 1.0 / 3.0, by6 ? kSixthLo : 2.0 * kSixthLo};
+    const double ahead = stage == 3 ? 1.0 : 0.5;
     auto skip = [](int fld) { return MATTER == kStaticMatter && fld == F_DIFFD; };
     double pv = __ldcs(&P.p[c]);
     double fv = stage == 1 ? 0.0 : __ldcs(&P.f[c]);
@@ -1543,12 +1551,17 @@ __device__ __forceinline__ void stage_body(const BoxGeom& geo, const Physics& ph
       }
       if (skip(fld)) continue;
       const double t = dt * S(cvslot(fld));
+      DivRange rg;
+      rg.numerator(t);
+      double q = by(t);
+      if (!rg.ok()) q = t / by.d;
+      if (t == 0.0) q = t;  // the zero's own sign
       double o;
       if (stage == 4) {
-        o = fcur + (t / 6.0 + pcur);
+        o = fcur + (q + pcur);
       } else {
-        __stcs(&P.f[(size_t)fld * N + c], fcur + t / fdiv);
-        o = pcur + t / odiv;
+        __stcs(&P.f[(size_t)fld * N + c], fcur + q);
+        o = pcur + t * ahead;
       }
       __stcs(&P.out[(size_t)fld * N + c], o);
       // at the last substep the new state is also the next step's first
