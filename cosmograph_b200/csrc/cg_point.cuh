@@ -99,6 +99,10 @@ struct DivRange {
   // every numerator zero or in [2^-e, 2^e]
   __device__ __forceinline__ bool within(unsigned e) const { return top < ((1023u + e) << 21) && low >= ((1023u - e) << 21); }
   __device__ __forceinline__ bool ok() const { return within(800); }
+  // one numerator: zero, or not in [2^-800, 2^800]
+  __device__ __forceinline__ static bool outside(double x) {
+    return ((unsigned)__double2hiint(x) << 1) - (223u << 21) >= (1600u << 21);
+  }
   // a divisor in [2^-100, 2^100]
   __device__ __forceinline__ static bool divisor_ok(double d) {
     return (((unsigned)__double2hiint(d) << 1) >> 21) - 923u <= 200u;

@@ -22,16 +22,17 @@
 //   out   a^{n+1} (n<4) or the new _p (n=4)
 // At n=4, norm receives the next step's first-substep input.
 //
-// Kernel shape.  A CTA owns a 4x4x8 (x,y,z) brick, one point per thread.
-// Phase 1 walks the stencil fields one at a time (a rolled loop, so the whole
-// CTA touches one field's halo region at a time and it stays in L1), computes
-// that field's derivatives at the thread's point and parks them in the
-// thread's column of a shared-memory slot array.  Phase 2 (the algebra of
-// set_bd_values and ev_*) reads the derivatives back from shared memory as it
-// needs them, so few values are live in registers at once.  Bricks whose
-// stencils never cross the periodic boundary use plain strided addressing;
-// the others wrap every tap.
+// Kernel shape.  A CTA owns a 4x6x16 (x,y,z) brick, one point per thread.
+// Phase 1 walks the stencil fields one at a time (a rolled loop over shared
+// memory halo tiles), computes that field's derivatives at the thread's point
+// and parks them in the thread's column of a shared-memory slot array.  Phase
+// 2 (the algebra of set_bd_values and ev_*) reads the derivatives back from
+// shared memory as it needs them, so few values are live in registers at once.
+// What bounds the kernel is the latency of dependent FP64 operations and of
+// the loads between them: twelve warps per SM, issuing 39 % of the cycles.
 #pragma once
+
+#include <type_traits>
 
 #include "cg_group.h"
 #include "cg_point.cuh"
@@ -85,64 +86,96 @@ template <int O>
 using TileG = tile::Geom<O, Brick, TileShape<O>::PITCH, TileShape<O>::ZO>;
 
 // Per-thread shared-memory slots (one column of kThreads doubles per slot).
+// The matter slots (dust: 4 divergences; scalar: 15 first derivatives) come
+// first, at negative slot numbers (Layout::MAT).
 enum : int {
-  S_DG = 0,           // d_I g_q           18  (later reused for Gamma_{I q})
-  S_T1 = 18,          // g^{kl} d_k d_l g_q  6
+  S_DG = 0,           // d_I g_q           18  (later the lowered symbols Gamma_{I q}, then right-hand sides)
+  S_T1 = 18,          // g^{kl} d_k d_l g_q  6  (then -1/2 of it + 1/2 of the d_J Gamma^K terms, then Ricci)
   S_DPHI = 24,        // d_I phi            3
   S_DDPHI = 27,       // d_I d_J phi        6
   S_DA = 33,          // d_I alpha          3
   S_DDA = 36,         // d_I d_J alpha      6
-  S_DK = 42,          // d_I K              3
-  S_DGAM = 45,        // d_J Gamma^K       9  (index 3*K + J)
-  S_SRC = 54,         // sources           11
-  S_G = 65,           // Gamma^I_q         18
-  S_MAT = 83,         // dust: 4 divergences; scalar: 15 first derivatives
-};
-// Phase 1 writes no slot in [S_SRC, S_MAT): that region holds the field tile
-// and its row offsets until phase 2 starts.
-constexpr int kTileSlot = S_SRC, kTileSlots = S_MAT - S_SRC;
-// Z4C: Z4c damping (USE_Z4c_DAMPING): the first derivatives of theta in
-// three more slots after the matter slots
-template <int MATTER, bool Z4C = false>
-struct Slots {
-  static constexpr int dth = S_MAT + (MATTER == kDust ? 4 : (MATTER == kScalar ? 15 : 0));
-  static constexpr int value = dth + (Z4C ? 3 : 0);
+  S_DK = 42,          // d_I K              3  (then the right-hand sides of Gamma^I)
+  S_END = 45,
+  S_DGAM = S_DPHI,    // d_J Gamma^K 9 (index 3*K + J) until they enter S_T1, before phi and alpha are differentiated
 };
 
 // What a launch of the point kernel does with the geometry it computes.
 enum Mode : int { kEvolve = 0, kConstraints = 1 };
-// constraint mode: d_d A_q after the matter slots (18)
-template <int MATTER, bool Z4C = false>
-struct SlotsC {
-  static constexpr int dA = Slots<MATTER, Z4C>::value;
-  static constexpr int value = dA + 18;
+
+// TMA boxes of the dust flux primitives for their divergence: for axis a the
+// brick extended by r along a only (z: to the row of the field tiles, which
+// starts at an aligned z).
+template <int O>
+struct FluxBox {
+  static constexpr int R = O / 2;
+  static constexpr int XB = (kBX + 2 * R) * kBY * kBZ;
+  static constexpr int YB = kBX * (kBY + 2 * R) * kBZ;
+  static constexpr int ZP = TileG<O>::TZ, ZB = kBX * kBY * ZP;
+  static constexpr int SIZE = 5 * (XB + YB + ZB);  // alpha*D, alpha*S_1..3 and v^a for each axis
 };
-// A second tile buffer after the slot array lets the TMA copy of the next
-// field overlap the derivatives of the current one.  Evolve mode, dust and
-// vacuum: two CTAs per SM still fit in shared memory (with Z4c's three more
-// slots they would not: one buffer).
-template <int O, int MATTER, int MODE, bool Z4C = false>
-struct TileBuffers {
-  static constexpr bool kTwo = MODE == kEvolve && MATTER != kScalar && !Z4C;
-  // dust also stages the x and z boxes of its flux primitives here (5 arrays
-  // each, flux_from_tiles)
-  static constexpr size_t kTile = TileG<O>::SIZE * sizeof(double);
-  static constexpr size_t kFluxX = 5 * (kBX + O) * kBY * kBZ * sizeof(double);
-  static constexpr size_t kFluxZ = 5 * kBX * kBY * TileG<O>::TZ * sizeof(double);
-  static constexpr size_t kNeed =
-      MATTER == kDust ? (kTile > kFluxX ? (kTile > kFluxZ ? kTile : kFluxZ) : (kFluxX > kFluxZ ? kFluxX : kFluxZ))
-                      : kTile;
-  static constexpr size_t kBytes = (kNeed + 127) / 128 * 128;
+struct FluxMaps {
+  CUtensorMap m[3];  // x, y and z boxes of the substep input's 7 flux-primitive arrays
 };
-// dynamic shared memory of a substep launch
-template <int O, int MATTER, int MODE, bool Z4C = false>
-constexpr size_t stage_smem() {
-  return sizeof(double) * kThreads * (MODE == kConstraints ? SlotsC<MATTER, Z4C>::value : Slots<MATTER, Z4C>::value) +
-         (TileBuffers<O, MATTER, MODE, Z4C>::kTwo ? TileBuffers<O, MATTER, MODE, Z4C>::kBytes : 0);
-}
-// two CTAs per SM (228 KB, 1 KB reserved per CTA, up to 1 KB of static shared memory)
-static_assert(2 * (stage_smem<8, kDust, kEvolve>() + 2048) <= 228 * 1024, "two dust CTAs fit on an SM");
-static_assert(2 * (stage_smem<8, kScalar, kEvolve, true>() + 2048) <= 228 * 1024, "two Z4c CTAs fit on an SM");
+
+// Shared memory of a CTA, in doubles.  Phase 1: the slots that survive it
+// (LIVE of them, after the matter slots), then the field tiles; the flux boxes
+// lie over the still empty slots and end where the first tile starts, so that
+// one round of copies brings all of them and the first field.  Phase 2: the
+// sources take the tiles' place.
+//
+// One CTA of twelve warps per SM.  Its warps run through the straight-line
+// algebra together, so that an instruction fetched once serves three warps of
+// a scheduler; three CTAs of four warps, each in another place of the code,
+// waited for instructions 1.5 cycles per issue (now 0.3).  256^3 dust, order 8,
+// ms a step: two CTAs of 128 threads with 254 registers 72.4, three of 128
+// 71.2, one of 256 66.8, two of 192 65.7, one of 384 62.6.  With the scratch
+// slots below (fewer spills), the register update eight fields at a time and
+// cheaper prefetches and waits it takes 55.3 (69.0 with 87 slots, two CTAs of
+// 128 and two buffers).
+template <int O, int MATTER, int MODE, bool Z4C = false, bool SHIFT = false>
+struct Layout {
+  // (constraint mode needs the scalar field's own derivatives only)
+  static constexpr int MATN = MATTER == kDust ? 4 : (MATTER == kScalar ? (MODE == kConstraints ? 3 : 15) : 0);
+  static constexpr int MAT = -MATN;                                 // first matter slot
+  static constexpr int dth = S_END;                                 // Z4c: d_I theta
+  static constexpr int dA = dth + (Z4C ? 3 : 0);                    // constraint mode: g^{Xd} d_d A_{XI}
+  static constexpr int LIVE = dA + (MODE == kConstraints ? 3 : 0);
+  static constexpr int SRC = LIVE;                                  // sources (Q_N), phase 2
+  static constexpr bool FLUX = MATTER == kDust && MODE == kEvolve;  // flux boxes are staged
+  static constexpr int kSlotEnd = (MATN + LIVE) * kThreads;
+  static constexpr int kFlux = MATN * kThreads;                     // flux boxes
+  static constexpr int kFluxEnd = FLUX ? kFlux + FluxBox<O>::SIZE : 0;
+  static constexpr int kTile = kSlotEnd > kFluxEnd ? kSlotEnd : kFluxEnd;  // first tile
+  static constexpr int kTileSize = TileG<O>::SIZE;
+  static constexpr int kRows = (TileG<O>::ROWS * (int)sizeof(int) + 127) / 128 * 16;  // row offsets of thread copies
+  static constexpr bool kRowsInGap = kTile - kSlotEnd >= kRows;
+  // static shared memory: up to 832 bytes (evolve), 2.8 KB (constraint mode's reductions)
+  static constexpr int kStatic = MODE == kConstraints ? 2816 : 832;
+  // Phase 2 scratch: values that stay live over the Ricci tensor's loop wait
+  // there in slots (a scalar field's derivatives leave ten, the rest lie after
+  // the sources), as many as a CTA's shared memory holds; the others stay in
+  // registers.
+  static constexpr int kScratchMat = MATTER == kScalar && MODE == kEvolve ? MATN - 5 : 0;
+  static constexpr int kScratchMax = 16;
+  static constexpr int kMaxDoubles = (227 * 1024 - kStatic) / (int)sizeof(double);
+  static constexpr int kScratchCap = kMaxDoubles / kThreads - (MATN + LIVE + Q_N) + kScratchMat;
+  static constexpr int NSCR = kScratchCap < kScratchMax ? kScratchCap : kScratchMax;
+  __host__ __device__ static constexpr int scratch(int n) { return n < kScratchMat ? MAT + 5 + n : SRC + Q_N + n - kScratchMat; }
+  static constexpr int total(int tiles) {
+    const int a = kTile + tiles * kTileSize + (kRowsInGap ? 0 : kRows);
+    const int b = (MATN + LIVE + Q_N + (NSCR > kScratchMat ? NSCR - kScratchMat : 0)) * kThreads;
+    return a > b ? a : b;
+  }
+  static constexpr bool fits(int tiles) { return total(tiles) <= kMaxDoubles; }
+  static constexpr bool TWO = fits(2);  // a second tile buffer
+  static constexpr int kRowOff = kRowsInGap ? kSlotEnd : kTile + (TWO ? 2 : 1) * kTileSize;
+  static constexpr size_t kBytes = sizeof(double) * (size_t)total(TWO ? 2 : 1);
+  static_assert(fits(1), "a CTA fits on an SM");
+  static_assert(kFlux % 16 == 0 && kTile % 16 == 0 && kTileSize % 16 == 0 && FluxBox<O>::XB % 16 == 0 &&
+                    FluxBox<O>::YB % 16 == 0 && FluxBox<O>::ZB % 16 == 0,
+                "TMA destinations are 128-byte aligned");
+};
 // per-block partial results of the constraint pass (see constraint_reduce)
 constexpr int kCPart = 27;
 
@@ -330,64 +363,76 @@ __device__ __forceinline__ void flux_sums(UF U, VF V, double (&out)[4]) {
 }
 
 // Fields copied into tiles in phase 1, in order: (constraint mode) A_q with
-// first derivatives; the metric components, phi and alpha with first and
-// second derivatives; K and Gamma^i with first derivatives; (scalar) phi, Pi,
-// psi_i with first derivatives.  With Z4c, theta (stored after the matter
-// fields) with first derivatives after Gamma^i.
+// first derivatives; the metric components with first and second, Gamma^i
+// with first, phi and alpha with first and second, K with first derivatives;
+// with Z4c, theta (stored after the matter fields), then (scalar) phi, Pi,
+// psi_i with first derivatives.
 template <int MATTER, int MODE, bool Z4C = false>
 struct Phase1 {
   static constexpr int NA = MODE == kConstraints ? 6 : 0;
   static constexpr int NZ = Z4C ? 1 : 0;
-  static constexpr int NS = MATTER == kScalar ? 5 : 0;
-  static constexpr int N = NA + 8 + 4 + NZ + NS;
+  static constexpr int NS = MATTER == kScalar ? (MODE == kConstraints ? 1 : 5) : 0;
+  static constexpr int GAM = NA + 6, PHI = NA + 9, K = NA + 11, TH = NA + 12, SC = TH + NZ;  // first of each kind
+  static constexpr int N = SC + NS;
   __device__ __forceinline__ static int field(int it) {
     if (it < NA) return F_A11 + it;
-    it -= NA;
-    if (it < 8) return it < 6 ? F_G11 + it : (it == 6 ? F_PHI : F_ALPHA);
-    it -= 8;
-    if (it < 4) return it == 0 ? F_K : F_GAM1 + it - 1;
-    it -= 4;
-    if (it < NZ) return NF<MATTER>::value;  // theta
-    it -= NZ;
-    return F_SPHI + it;
+    if (it < GAM) return F_G11 + it - NA;
+    if (it < PHI) return F_GAM1 + it - GAM;
+    if (it < K) return it == PHI ? F_PHI : F_ALPHA;
+    if (it == K) return F_K;
+    if (it < SC) return NF<MATTER>::value;  // theta
+    return F_SPHI + it - SC;
   }
 };
 
 // Phase 1: every derivative the point needs, parked in shared memory.  One
-// field at a time is copied into the tile (the next one is fetched into
-// registers, or into L2 on the TMA path, meanwhile); all threads of the CTA
-// take part.
+// field at a time is copied into a tile; all threads of the CTA take part.
 //
 // The copies: by TMA when tmap is set (a brick whose halo lies inside the
-// box), else by the threads' own loads with periodic wrap.  Returns false (the
-// same value in every thread) when a TMA copy did not complete within
-// ph.tma_wait cycles; the status word then carries kStatusTileTimeout64.  A
-// late copy is still waited for (tma::wait_drain), so that no copy is in
-// flight when a buffer is reused or the CTA leaves; after a copy that never
-// lands the CTA issues no more.
-template <int O, int MATTER, int MODE, bool Z4C>
-__device__ __forceinline__ void field_derivatives(int it, const tile::Taps<TileG<O>, double>& t, const Physics& ph,
-                                                  const double gi[6], double* sl);
-
+// box; the next field into the second tile buffer, or, with one buffer, into
+// L2 meanwhile), else by the threads' cp.async with periodic wrap.  With fm
+// (dust) the boxes of the flux primitives come first, in one round with the
+// first tile.  Returns false (the same value in every thread) when a TMA copy
+// did not complete within ph.tma_wait cycles; the status word then carries
+// kStatusTileTimeout64.  A late copy is still waited for (tma::wait_drain),
+// so that no copy is in flight when a buffer is reused or the CTA leaves;
+// after a copy that never lands the CTA issues no more.
 //
-// bar[0] (and bar[1] with two buffers) are the buffers' mbarriers; bit b of
-// phase is the parity bar[b] completes next.
-template <int O, int MATTER, int MODE, bool Z4C = false>
-__device__ __forceinline__ bool derivatives(const double* __restrict__ a, int N, const Physics& ph, const double gi[6],
-                                            double* sl, double* tl, double* tl2, const int* rowoff, int tid, int x0,
-                                            int y0, int z0, int nz, int cc, const CUtensorMap* tmap, uint64_t* bar,
-                                            unsigned& phase, unsigned* status) {
+// bar[0], bar[1]: mbarriers of the tile buffers, bar[2] of the flux boxes; bit
+// b of phase is the parity bar[b] completes next.  (tx, ty, tz): the thread's
+// point in the brick.
+template <int O, int MATTER, int MODE, bool Z4C, bool SHIFT>
+__device__ __forceinline__ void field_derivatives(int it, const tile::Taps<TileG<O>, double>& t, const Physics& ph,
+                                                  const double g[6], const double gi[6], double* sl);
+template <int O, class AxisOf>
+__device__ __forceinline__ void flux_divergences(AxisOf axis, const Physics& ph, double* mat);
+// taps of one axis in its five staged boxes of len values, stride st
+struct BoxAxis {
+  const double* u;
+  int len, st;
+  __device__ __forceinline__ double operator()(int m, int n) const { return u[m * len + n * st]; }
+};
+
+template <int O, int MATTER, int MODE, bool Z4C, bool SHIFT>
+__device__ __forceinline__ bool derivatives(const double* __restrict__ a, int N, const Physics& ph, const double g[6],
+                                            const double gi[6], double* smem, double* sl, int tid, int x0, int y0,
+                                            int z0, int tx, int ty, int tz, int nz, const CUtensorMap* tmap,
+                                            const FluxMaps* fm, uint64_t* bar, unsigned& phase, unsigned* status) {
   using PF = Phase1<MATTER, MODE, Z4C>;
+  using L = Layout<O, MATTER, MODE, Z4C, SHIFT>;
   using G = TileG<O>;
-  constexpr bool TWO = TileBuffers<O, MATTER, MODE, Z4C>::kTwo;
-  constexpr unsigned kBytes = (unsigned)(G::SIZE * sizeof(double));
+  constexpr bool TWO = L::TWO;
+  double* tl = smem + L::kTile;
+  double* tl2 = tl + (TWO ? L::kTileSize : 0);
+  const int* rowoff = reinterpret_cast<const int*>(smem + L::kRowOff);
+  const int cc = tile::centre<G>(tx, ty, tz);
   // TMA: field it into buffer it % 2 (one buffer: 0), field it + 1 into L2;
   // thread 0 copies, every thread notes the buffer's copy as pending
   unsigned pending = 0;
   auto issue = [&](int it) {
     const int b = TWO ? (it & 1) : 0;
     if (tid == 0) {
-      tma::arrive_expect_tx(bar + b, kBytes);
+      tma::arrive_expect_tx(bar + b, (unsigned)(G::SIZE * sizeof(double)));
       tma::load_4d(b ? tl2 : tl, tmap, z0 - G::ZO, y0 - G::R, x0 - G::R, PF::field(it), bar + b);
       if (it + 1 < PF::N) tma::prefetch_4d(tmap, z0 - G::ZO, y0 - G::R, x0 - G::R, PF::field(it + 1));
     }
@@ -406,52 +451,79 @@ __device__ __forceinline__ bool derivatives(const double* __restrict__ a, int N,
     else phase ^= 1u << b;
   };
   const bool by_tma = tmap != nullptr;
-  tile::Loader<G, Brick, double> ld;
-  tile::AsyncLoader<G, Brick> ald;
+  tile::AsyncLoader<G, Brick, double> ald;
   if (by_tma) {
-    if (TWO) {
-      tma::fence_proxy_async();  // this thread's shared-memory accesses come before the copy's writes
-      __syncthreads();
-      issue(0);
+    tma::fence_proxy_async();  // this thread's shared-memory accesses come before the copies' writes
+    __syncthreads();
+    if constexpr (L::FLUX) {
+      if (fm) {
+        using FB = FluxBox<O>;
+        double* box = smem + L::kFlux;
+        if (tid == 0) {
+          tma::arrive_expect_tx(bar + 2, (unsigned)(FB::SIZE * sizeof(double)));
+          for (int ax = 0; ax < 3; ++ax) {
+            const int len = ax == 0 ? FB::XB : (ax == 1 ? FB::YB : FB::ZB);
+            for (int q = 0; q < 5; ++q, box += len)  // alpha*D, alpha*S_1..3, then v^a
+              tma::load_4d(box, &fm->m[ax], z0 - (ax == 2 ? G::ZO : 0), y0 - (ax == 1 ? FB::R : 0),
+                           x0 - (ax == 0 ? FB::R : 0), q < 4 ? P_AD + q : P_V1 + ax, bar + 2);
+          }
+        }
+        pending |= 4u;
+      }
     }
-  } else if (TWO) {
-    // two buffers: cp.async copies of field it + 1 run while field it is differentiated
+    issue(0);
+    if constexpr (L::FLUX) {
+      if (fm) {
+        using FB = FluxBox<O>;
+        const double* box = smem + L::kFlux;
+        wait(2);
+        flux_divergences<O>(
+            [&](int ax) {
+              const int c = ax == 0   ? ((tx + FB::R) * kBY + ty) * kBZ + tz
+                            : ax == 1 ? 5 * FB::XB + (tx * (kBY + 2 * FB::R) + ty + FB::R) * kBZ + tz
+                                      : 5 * (FB::XB + FB::YB) + (tx * kBY + ty) * FB::ZP + tz + G::ZO;
+              return BoxAxis{box + c, ax == 0 ? FB::XB : (ax == 1 ? FB::YB : FB::ZB),
+                             ax == 0 ? kBY * kBZ : (ax == 1 ? kBZ : 1)};
+            },
+            ph, sl + L::MAT * kThreads);
+      }
+    }
+  } else {
     ald.init(tid, z0, nz);
     ald.issue(tl, a + (size_t)PF::field(0) * N, rowoff);
-  } else {
-    ld.init(tid, z0, nz);
-    ld.fetch(a + (size_t)PF::field(0) * N, rowoff);
   }
   // one loop (and one copy of the derivative code) for both kinds of copy
 #pragma unroll 1
   for (int it = 0; it < PF::N; ++it) {
-    int b = 0;
+    const int b = TWO ? (it & 1) : 0;
+    // the buffer that the next copy writes has been read (first pass: the flux boxes, which the slots overwrite)
     if (by_tma) {
       tma::fence_proxy_async();
-      lost = __syncthreads_or(lost);  // the buffer the next copy writes has been read
+      lost = __syncthreads_or(lost);
       if (!lost) {
-        if (!TWO) issue(it);
-        else if (it + 1 < PF::N) issue(it + 1);
+        if (TWO) {
+          if (it + 1 < PF::N) issue(it + 1);
+        } else if (it > 0) {
+          issue(it);
+        }
       }
-      b = TWO ? (it & 1) : 0;
       wait(b);
-    } else if (TWO) {
-      __syncthreads();  // the buffer the next copies write has been read
-      if (it + 1 < PF::N) {
-        ald.issue((it + 1) & 1 ? tl2 : tl, a + (size_t)PF::field(it + 1) * N, rowoff);
-        tile::cp_async_wait<1>();  // this thread's copies of field it have landed
+    } else {
+      __syncthreads();
+      if (TWO) {
+        if (it + 1 < PF::N) {
+          ald.issue((it + 1) & 1 ? tl2 : tl, a + (size_t)PF::field(it + 1) * N, rowoff);
+          tile::cp_async_wait<1>();  // this thread's copies of field it have landed
+        } else {
+          tile::cp_async_wait<0>();
+        }
       } else {
+        if (it > 0) ald.issue(tl, a + (size_t)PF::field(it) * N, rowoff);
         tile::cp_async_wait<0>();
       }
       __syncthreads();  // and every other thread's
-      b = it & 1;
-    } else {
-      __syncthreads();  // the previous tile has been read
-      ld.store(tl);
-      __syncthreads();
-      if (it + 1 < PF::N) ld.fetch(a + (size_t)PF::field(it + 1) * N, rowoff);
     }
-    field_derivatives<O, MATTER, MODE, Z4C>(it, tile::Taps<G, double>{b ? tl2 : tl, cc}, ph, gi, sl);
+    field_derivatives<O, MATTER, MODE, Z4C, SHIFT>(it, tile::Taps<G, double>{b ? tl2 : tl, cc}, ph, g, gi, sl);
   }
   if (by_tma) {
     wait(0);  // after a lost copy: the other buffer's copy in flight
@@ -463,175 +535,131 @@ __device__ __forceinline__ bool derivatives(const double* __restrict__ a, int N,
 }
 
 // the derivatives of phase-1 field `it` from its tile, into the slots
-template <int O, int MATTER, int MODE, bool Z4C>
+template <int O, int MATTER, int MODE, bool Z4C, bool SHIFT>
 __device__ __forceinline__ void field_derivatives(int it, const tile::Taps<TileG<O>, double>& t, const Physics& ph,
-                                                  const double gi[6], double* sl) {
+                                                  const double g[6], const double gi[6], double* sl) {
   using PF = Phase1<MATTER, MODE, Z4C>;
-  {
-    if (it >= PF::NA && it < PF::NA + 8) {
-      // calculate_dgamma / calculate_ddgamma / calculate_dalpha_dphi
-      // (bssn.cc:480-521).  For g_q the second derivatives are contracted at
-      // once with the inverse metric (BSSN_CALCULATE_RICCI_UNITARY_TERM1,
-      // bssn_macros.h:248-249, summed over (k,l) in the reference's order).
-      // The nine sums first and their divisions in one batch: independent
-      // chains in one block, where a choice of the division per sum kept
-      // them apart.
+  using L = Layout<O, MATTER, MODE, Z4C, SHIFT>;
+  auto S = [&](int s) -> double& { return sl[s * kThreads]; };
+  if ((it >= PF::NA && it < PF::GAM) || (it >= PF::PHI && it < PF::K)) {
+    // calculate_dgamma / calculate_ddgamma / calculate_dalpha_dphi
+    // (bssn.cc:480-521).  For g_q the second derivatives are contracted at
+    // once with the inverse metric (BSSN_CALCULATE_RICCI_UNITARY_TERM1,
+    // bssn_macros.h:248-249, summed over (k,l) in the reference's order).
+    // The nine sums first and their divisions in one batch: independent
+    // chains in one block, where a choice of the division per sum kept
+    // them apart.
+    double s[9] = {s1<O>(t, 0), s1<O>(t, 1), s1<O>(t, 2), s2<O>(t, 0),    s2<O>(t, 1),
+                   s2<O>(t, 2), sm<O>(t, 0, 1), sm<O>(t, 0, 2), sm<O>(t, 1, 2)};
+    div_dx<9, 3>(s, ph);
+    const double h11 = s[3], h22 = s[4], h33 = s[5], h12 = s[6], h13 = s[7], h23 = s[8];
+    if (it < PF::GAM) {
       const int q = it - PF::NA;
-      double s[9] = {s1<O>(t, 0), s1<O>(t, 1), s1<O>(t, 2), s2<O>(t, 0),    s2<O>(t, 1),
-                     s2<O>(t, 2), sm<O>(t, 0, 1), sm<O>(t, 0, 2), sm<O>(t, 1, 2)};
-      div_dx<9, 3>(s, ph);
-      const double h11 = s[3], h22 = s[4], h33 = s[5], h12 = s[6], h13 = s[7], h23 = s[8];
-      if (q < 6) {
-        sl[(S_DG + 0 * 6 + q) * kThreads] = s[0];
-        sl[(S_DG + 1 * 6 + q) * kThreads] = s[1];
-        sl[(S_DG + 2 * 6 + q) * kThreads] = s[2];
-        double u = gi[0] * h11;
-        u = u + gi[1] * h12;
-        u = u + gi[2] * h13;
-        u = u + gi[1] * h12;
-        u = u + gi[3] * h22;
-        u = u + gi[4] * h23;
-        u = u + gi[2] * h13;
-        u = u + gi[4] * h23;
-        u = u + gi[5] * h33;
-        sl[(S_T1 + q) * kThreads] = u;
-      } else {
-        const int b1 = q == 6 ? S_DPHI : S_DA, b2 = q == 6 ? S_DDPHI : S_DDA;
-        sl[(b1 + 0) * kThreads] = s[0];
-        sl[(b1 + 1) * kThreads] = s[1];
-        sl[(b1 + 2) * kThreads] = s[2];
-        sl[(b2 + 0) * kThreads] = h11;
-        sl[(b2 + 1) * kThreads] = h12;
-        sl[(b2 + 2) * kThreads] = h13;
-        sl[(b2 + 3) * kThreads] = h22;
-        sl[(b2 + 4) * kThreads] = h23;
-        sl[(b2 + 5) * kThreads] = h33;
-      }
+      S(S_DG + 0 * 6 + q) = s[0];
+      S(S_DG + 1 * 6 + q) = s[1];
+      S(S_DG + 2 * 6 + q) = s[2];
+      double u = gi[0] * h11;
+      u = u + gi[1] * h12;
+      u = u + gi[2] * h13;
+      u = u + gi[1] * h12;
+      u = u + gi[3] * h22;
+      u = u + gi[4] * h23;
+      u = u + gi[2] * h13;
+      u = u + gi[4] * h23;
+      u = u + gi[5] * h33;
+      S(S_T1 + q) = u;
     } else {
-      // first derivatives only, into three slots
-      int b;
-      if (it < PF::NA) {
-        b = SlotsC<MATTER, Z4C>::dA + 3 * it;  // d_d A_q for the momentum constraint (BSSN_MI, bssn_macros.h:498-500)
-      } else if (it < PF::NA + 12) {
-        // K and Gamma^K (calculate_dK, bssn.cc:529-535; the d_J Gamma^K of
-        // BSSN_CALCULATE_RICCI_UNITARY_TERM2, bssn_macros.h:251-252)
-        const int q = it - PF::NA - 8;
-        b = q == 0 ? S_DK : S_DGAM + 3 * (q - 1);
-      } else if (Z4C && it == PF::NA + 12) {
-        b = Slots<MATTER, Z4C>::dth;  // calculate_dtheta (bssn.cc:537-544)
-      } else {
-        b = S_MAT + 3 * (it - PF::NA - 12 - PF::NZ);  // Scalar::getScalarData (scalar.cc:109-127): phi, Pi, psi1..3
-      }
-      double g[3];
-      grad<O>(t, ph, g);
-#pragma unroll
-      for (int d = 0; d < 3; ++d) sl[(b + d) * kThreads] = g[d];
+      const int b1 = it == PF::PHI ? S_DPHI : S_DA, b2 = it == PF::PHI ? S_DDPHI : S_DDA;
+      S(b1 + 0) = s[0];
+      S(b1 + 1) = s[1];
+      S(b1 + 2) = s[2];
+      S(b2 + 0) = h11;
+      S(b2 + 1) = h12;
+      S(b2 + 2) = h13;
+      S(b2 + 3) = h22;
+      S(b2 + 4) = h23;
+      S(b2 + 5) = h33;
     }
+    return;
+  }
+  // first derivatives only, into three slots
+  int b;
+  if (it < PF::NA) b = S_DGAM;                             // d_d A_q
+  else if (it < PF::PHI) b = S_DGAM + 3 * (it - PF::GAM);  // d_J Gamma^K
+  else if (it == PF::K) b = S_DK;                          // calculate_dK, bssn.cc:529-535
+  else if (Z4C && it == PF::TH) b = L::dth;                // calculate_dtheta (bssn.cc:537-544)
+  else b = L::MAT + 3 * (it - PF::SC);                     // Scalar::getScalarData (scalar.cc:109-127): phi, Pi, psi1..3
+  double d[3];
+  grad<O>(t, ph, d);
+#pragma unroll
+  for (int x = 0; x < 3; ++x) S(b + x) = d[x];
+  if (it < PF::NA) {
+    // g^{Xd} d_d A_{XI} of the momentum constraint (BSSN_MI, bssn_macros.h:
+    // 498-500), summed with X slow: the order in which A_11, A_12, ... come
+#pragma unroll
+    for (int q = 0; q < 6; ++q) {
+      if (q != it) continue;
+      const int X = q < 3 ? 0 : (q < 5 ? 1 : 2), I = q < 3 ? q : (q < 5 ? q - 2 : 2);  // sym(X, I) = q
+#pragma unroll
+      for (int two = 0; two < (X == I ? 1 : 2); ++two) {
+        const int to = two ? X : I, from = two ? I : X;  // A_{from to}
+        double t = from == 0 ? 0.0 : S(L::dA + to);
+#pragma unroll
+        for (int x = 0; x < 3; ++x) t = (from == 0 && x == 0) ? gi[sym(from, x)] * d[x] : t + gi[sym(from, x)] * d[x];
+        S(L::dA + to) = t;
+      }
+    }
+  }
+  if (it == PF::PHI - 1) {
+    // all of d_J Gamma^K: BSSN_CALCULATE_RICCI_UNITARY_TERM2 (bssn_macros.h:
+    // 251-252) joins term 1, as the first two terms of the reference's sum;
+    // phi and alpha then take the slots
+    double gm[6], dG[9], B[3][3];
+#pragma unroll
+    for (int m = 0; m < 6; ++m) gm[m] = (m == 0 || m == 3 || m == 5) ? g[m] + 1.0 : g[m];
+#pragma unroll
+    for (int m = 0; m < 9; ++m) dG[m] = S(S_DGAM + m);
+#pragma unroll
+    for (int I = 0; I < 3; ++I)
+#pragma unroll
+      for (int J = 0; J < 3; ++J) B[I][J] = gm[sym(0, I)] * dG[J] + gm[sym(1, I)] * dG[3 + J] + gm[sym(2, I)] * dG[6 + J];
+#pragma unroll
+    for (int I = 0; I < 3; ++I)
+#pragma unroll
+      for (int J = I; J < 3; ++J) S(S_T1 + sym(I, J)) = -0.5 * S(S_T1 + sym(I, J)) + 0.5 * (B[I][J] + B[J][I]);
   }
 }
 
 // Dust flux divergences d_i(alpha D v^i), d_i(alpha S_m v^i) (dust.cc:203-224)
-// from the stored flux primitives, taps read from global memory.
-template <int O, class T>
-__device__ __forceinline__ void flux_divergences(const T& t, const double* __restrict__ fp, int N, const Physics& ph,
-                                                 double* sl) {
+// into the matter slots, one axis at a time in a rolled loop; axis(a): the taps
+// of axis a, (m, n) -> the value at offset n of alpha*D, alpha*S_1..3 (m < 4)
+// or v^a (m = 4).
+template <int O, class AxisOf>
+__device__ __forceinline__ void flux_divergences(AxisOf axis, const Physics& ph, double* mat) {
   double div[4] = {0.0, 0.0, 0.0, 0.0};
-#pragma unroll
+#pragma unroll 1
   for (int a = 0; a < 3; ++a) {
-    const double* v = fp + (size_t)(P_V1 + a) * N;
+    const auto t = axis(a);
     double s[4];
-    flux_sums<O>([&](int m, int n) { return __ldg(fp + (size_t)(P_AD + m) * N + t.ax(a, n)); },
-                 [&](int n) { return __ldg(v + t.ax(a, n)); }, s);
+    flux_sums<O>([&](int m, int n) { return t(m, n); }, [&](int n) { return t(4, n); }, s);
     div_dx<4, 4>(s, ph);
 #pragma unroll
     for (int m = 0; m < 4; ++m) div[m] = a == 0 ? s[m] : div[m] + s[m];
   }
 #pragma unroll
-  for (int m = 0; m < 4; ++m) sl[(S_MAT + m) * kThreads] = div[m];
+  for (int m = 0; m < 4; ++m) mat[m * kThreads] = div[m];
 }
-
-// TMA boxes of the dust flux primitives for their divergence: for axis a the
-// brick extended by r along a only (x: (4+2r) x 2 x 16, y: 4 x (2+2r) x 16,
-// z: 4 x 2 x the tile row of the field tiles, starting at an aligned z).
+// taps of one axis in global memory: u alpha*D at the point, v its v^a, off[]
+// the (periodic) offsets -R..-1, 1..R
 template <int O>
-struct FluxBox {
-  static constexpr int R = O / 2;
-  static constexpr int XB = (kBX + 2 * R) * kBY * kBZ;
-  static constexpr int YB = kBX * (kBY + 2 * R) * kBZ;
-  static constexpr int ZP = TileG<O>::TZ, ZB = kBX * kBY * ZP;
-};
-struct FluxMaps {
-  CUtensorMap m[3];  // x, y and z boxes of the substep input's 7 flux-primitive arrays
-};
-
-// Dust flux divergences of a brick inside the box from TMA boxes: x boxes
-// into tl2, y boxes into tl, then z boxes into tl2; the sum over axes in the
-// order of flux_divergences.  All threads of the CTA take part.
-// (tx, ty, tz): the thread's point in the brick
-template <int O>
-__device__ __forceinline__ bool flux_from_tiles(const FluxMaps* fm, double* tl, double* tl2, int tid, int x0, int y0,
-                                                int z0, const Physics& ph, double* sl, uint64_t* bar,
-                                                unsigned& phase, int tx, int ty, int tz) {
-  using FB = FluxBox<O>;
-  constexpr int R = FB::R;
-  // every staging area fits its buffer: x and z boxes in the second tile
-  // buffer, y boxes in the first (the phase-2-only slot columns)
-  static_assert(5 * FB::XB * sizeof(double) <= TileBuffers<O, kDust, kEvolve>::kBytes, "x boxes fit");
-  static_assert(5 * FB::ZB * sizeof(double) <= TileBuffers<O, kDust, kEvolve>::kBytes, "z boxes fit");
-  static_assert(5 * FB::YB * sizeof(double) <= (size_t)kTileSlots * kThreads * sizeof(double), "y boxes fit");
-  // as in derivatives: bounded waits that let late copies land; after a lost
-  // copy no more copies, the ones in flight waited for
-  bool ok = true, lost = false;
-  unsigned pending = 0;
-  auto wait = [&](int b) {
-    if (!(pending & (1u << b))) return;
-    const int w = tma::wait_drain(bar + b, (phase >> b) & 1u, ph.tma_wait);
-    ok = ok && w == 0;
-    pending &= ~(1u << b);
-    if (w == 2) lost = true;
-    else phase ^= 1u << b;
-  };
-  auto load5 = [&](int a, double* dst, uint64_t* b, int len) {
-    tma::arrive_expect_tx(b, (unsigned)(5 * len * sizeof(double)));
-    const int cx = x0 - (a == 0 ? R : 0), cy = y0 - (a == 1 ? R : 0);
-    const int cz = z0 - (a == 2 ? TileG<O>::ZO : 0);
-    for (int q = 0; q < 5; ++q)  // alpha*D, alpha*S_1..3, then v^a
-      tma::load_4d(dst + (size_t)q * len, &fm->m[a], cz, cy, cx, q < 4 ? P_AD + q : P_V1 + a, b);
-  };
-  tma::fence_proxy_async();
-  __syncthreads();  // the field tiles have been read
-  if (tid == 0) {
-    load5(0, tl2, bar + 1, FB::XB);
-    load5(1, tl, bar, FB::YB);
+struct GlobalAxis {
+  const double *u, *v;
+  size_t N;
+  int off[O];
+  __device__ __forceinline__ double operator()(int m, int n) const {
+    return __ldg((m < 4 ? u + m * N : v) + off[n < 0 ? n + O / 2 : O / 2 + n - 1]);
   }
-  // the term along one axis from its five boxes at u (the m-th array at
-  // u + m len, v^a after them), centre c, tap stride s
-  double div[4], q[4];
-  auto term = [&](const double* u, int len, int c, int s) {
-    flux_sums<O>([&](int m, int n) { return u[m * len + c + n * s]; }, [&](int n) { return u[4 * len + c + n * s]; }, q);
-    div_dx<4, 4>(q, ph);
-  };
-  pending = 3u;
-  wait(1);
-  term(tl2, FB::XB, ((tx + R) * kBY + ty) * kBZ + tz, kBY * kBZ);
-#pragma unroll
-  for (int m = 0; m < 4; ++m) div[m] = q[m];
-  tma::fence_proxy_async();
-  lost = __syncthreads_or(lost);  // the x boxes have been read
-  if (!lost) {
-    if (tid == 0) load5(2, tl2, bar + 1, FB::ZB);
-    pending |= 2u;
-  }
-  wait(0);
-  term(tl, FB::YB, (tx * (kBY + 2 * R) + ty + R) * kBZ + tz, kBZ);
-#pragma unroll
-  for (int m = 0; m < 4; ++m) div[m] = div[m] + q[m];
-  wait(1);
-  term(tl2, FB::ZB, (tx * kBY + ty) * FB::ZP + tz + TileG<O>::ZO, 1);
-#pragma unroll
-  for (int m = 0; m < 4; ++m) sl[(S_MAT + m) * kThreads] = div[m] + q[m];
-  return __syncthreads_and(ok && !lost);
-}
+};
 
 // Kreiss-Oliger dissipation of one field at (i, j, k) (utils/math.h:36-72;
 // the reference defines it for stencil orders 2 and 8 only): the sixth
@@ -715,17 +743,14 @@ __device__ __forceinline__ void stage_body(const BoxGeom& geo, const Physics& ph
   constexpr int F_BETA = NF<MATTER>::value + (Z4C ? 1 : 0), F_AUXB = F_BETA + 3, F_EXPN = F_BETA + 6;
   constexpr int NFLD = NF<MATTER>::value + (Z4C ? 1 : 0) + (SHIFT ? 7 : 0);
   static_assert(!SHIFT || MODE == kEvolve, "constraint statistics do not read the shift");
-  constexpr int NSLOT = MODE == kConstraints ? SlotsC<MATTER, Z4C>::value : Slots<MATTER, Z4C>::value;
+  using L = Layout<O, MATTER, MODE, Z4C, SHIFT>;
+  constexpr int MAT = L::MAT, SRC = L::SRC;
   // Z4c damping amplitudes (cosmo_macros.h:94-100)
   constexpr double k1 = Z4C ? 0.5 : 0.0, k2 = Z4C ? 0.1 : 0.0;
-  static_assert(NSLOT >= S_MAT, "the tile region lies inside the slot array");
-  static_assert(TileG<O>::SIZE * sizeof(double) + TileG<O>::ROWS * sizeof(int) <=
-                    (size_t)kTileSlots * kThreads * sizeof(double),
-                "tile and row offsets fit the phase-2-only slots");
   constexpr int R = O / 2;
   extern __shared__ __align__(128) double smem[];  // 128-byte aligned: TMA destinations
   const int tid = threadIdx.x + kBZ * (threadIdx.y + kBY * threadIdx.z);
-  double* sl = smem + tid;  // this thread's slot column
+  double* sl = smem + L::MATN * kThreads + tid;  // this thread's slot column
   auto S = [&](int s) -> double& { return sl[s * kThreads]; };
 
   const int k0 = cz * kBZ + threadIdx.x;
@@ -740,16 +765,32 @@ __device__ __forceinline__ void stage_body(const BoxGeom& geo, const Physics& ph
   const int N = geo.pts;
   const int c = (i * geo.ny + j) * geo.nz + k;
   const double* __restrict__ a = P.in;
-  auto C = [&](int f) { return a[(size_t)f * N + c]; };
+  // element c of field f of a block: the field's address is the same for the
+  // whole CTA, the thread's part a 32-bit byte offset (fields of at most 2^28
+  // points: a box's registers of more would not fit the GPU)
+  const unsigned c8 = (unsigned)c * 8u;
+  auto fat = [&](auto* block, int f) { return reinterpret_cast<decltype(block)>((uintptr_t)(block + (size_t)f * N) + c8); };
+  auto C = [&](int f) { return *fat(a, f); };
+  const int x0 = cx * kBX, y0 = cy * kBY, z0 = cz * kBZ;
   // The epilogue's register reads (_p, _f) are issued long after this point;
   // warm L2 with them now.  Those reads and every epilogue write are
   // single-use streams (ld/st .cs, evict first), which leaves L2 to the
-  // neighbouring bricks' tile rows.
+  // neighbouring bricks' tile rows.  One prefetch per 32-byte sector of the
+  // brick's rows (rows that do not start on a sector reach into one more): a
+  // quarter of a prefetch per element's instructions.
   if (MODE == kEvolve) {
+    constexpr int SEC = kBZ / 4 + 1, PER = kBX * kBY * SEC, GRP = kThreads / PER;  // a field's sectors, fields at a time
+    if (tid < GRP * PER) {
+      const int b = tid % PER, row = b / SEC;
+      const int x = min(x0 + row / kBY, geo.nx - 1), y = min(y0 + row % kBY, geo.ny - 1);
+      const int z = min(z0 + 4 * (b % SEC), min(z0 + kBZ, geo.nz) - 1);
+      const size_t at = (size_t)(tid / PER) * N + ((x * geo.ny + y) * geo.nz + z);
 #pragma unroll 1
-    for (int f = 0; f < NFLD; ++f) {
-      asm volatile("prefetch.global.L2 [%0];" :: "l"(P.p + (size_t)f * N + c));
-      if (stage > 1) asm volatile("prefetch.global.L2 [%0];" :: "l"(P.f + (size_t)f * N + c));
+      for (int reg = 0; reg < (stage > 1 ? 2 : 1); ++reg) {
+        const double* q = (reg ? P.f : P.p) + at;
+#pragma unroll 4
+        for (int f = tid / PER; f < NFLD; f += GRP, q += (size_t)GRP * N) asm volatile("prefetch.global.L2 [%0];" :: "l"(q));
+      }
     }
   }
 
@@ -760,47 +801,39 @@ __device__ __forceinline__ void stage_body(const BoxGeom& geo, const Physics& ph
   inv_metric(g, gi);
 
   // ---- phase 1: derivatives into shared memory ---------------------------------
-  const int x0 = cx * kBX, y0 = cy * kBY, z0 = cz * kBZ;
   bool flux_tiles = false;  // the dust flux divergences came from TMA boxes
   {
     using G = TileG<O>;
-    double* tl = smem + kTileSlot * kThreads;
-    int* rowoff = reinterpret_cast<int*>(tl + G::SIZE);
     // TMA when the brick's halo lies inside the box (no wrap)
     const bool by_tma = tmap && tma_ok && x0 >= G::R && x0 + kBX + G::R <= geo.nx && y0 >= G::R &&
                         y0 + kBY + G::R <= geo.ny && z0 >= G::ZO && z0 + kBZ + G::R <= geo.nz;
     if (!by_tma) {
-      tile::row_offsets<G, Brick>(x0, y0, geo.nx, geo.ny, geo.nz, tid, rowoff);
+      tile::row_offsets<G, Brick>(x0, y0, geo.nx, geo.ny, geo.nz, tid, reinterpret_cast<int*>(smem + L::kRowOff));
       __syncthreads();  // every warp reads every row offset
     }
+    flux_tiles = L::FLUX && fmaps && by_tma;
     // after a copy timed out the CTA copies by threads (the barrier's phase is unknown)
-    double* tl2 = TileBuffers<O, MATTER, MODE, Z4C>::kTwo ? smem + NSLOT * kThreads : nullptr;
-    tma_ok = derivatives<O, MATTER, MODE, Z4C>(a, N, ph, gi, sl, tl, tl2, rowoff, tid, x0, y0, z0, geo.nz,
-                                          tile::centre<G>(threadIdx.z, threadIdx.y, threadIdx.x),
-                                          by_tma ? tmap : nullptr, bar, phase, P.status) &&
+    tma_ok = derivatives<O, MATTER, MODE, Z4C, SHIFT>(a, N, ph, g, gi, smem, sl, tid, x0, y0, z0, threadIdx.z,
+                                                      threadIdx.y, threadIdx.x, geo.nz, by_tma ? tmap : nullptr,
+                                                      flux_tiles ? fmaps : nullptr, bar, phase, P.status) &&
              tma_ok;
-    if constexpr (MATTER == kDust && MODE == kEvolve && TileBuffers<O, MATTER, MODE, Z4C>::kTwo) {
-      flux_tiles = fmaps && by_tma && tma_ok;
-      if (flux_tiles) {
-        tma_ok = flux_from_tiles<O>(fmaps, tl, tl2, tid, x0, y0, z0, ph, sl, bar, phase, threadIdx.z, threadIdx.y,
-                                    threadIdx.x);
-        if (!tma_ok && tid == 0) atomicOr(P.status, kStatusTileTimeout64);
-      }
-    }
-    __syncthreads();  // the tile region becomes slots again
+    __syncthreads();  // the tiles become slots again
   }
   if (MODE == kEvolve && !live) return;  // no CTA-wide synchronisation after this point
   if (!flux_tiles) {
-    const bool interior = x0 >= R && x0 + kBX + R <= geo.nx && y0 >= R && y0 + kBY + R <= geo.ny && z0 >= R &&
-                          z0 + kBZ + R <= geo.nz;
     // the dust flux divergences of bricks that did not take them from TMA
     // boxes: taps from global memory
-    if (MATTER == kDust) {
-      if (interior) flux_divergences<O>(Taps<false>{i, j, k, geo.nx, geo.ny, geo.nz, geo.ny * geo.nz, geo.nz, c},
-                                        P.fp_in, N, ph, sl);
-      else flux_divergences<O>(Taps<true>{i, j, k, geo.nx, geo.ny, geo.nz, geo.ny * geo.nz, geo.nz, c}, P.fp_in, N,
-                               ph, sl);
-    }
+    if (MATTER == kDust && MODE == kEvolve)
+      flux_divergences<O>(
+          [&](int ax) {
+            const int at = ax == 0 ? i : (ax == 1 ? j : k), n = ax == 0 ? geo.nx : (ax == 1 ? geo.ny : geo.nz);
+            const int st = ax == 0 ? geo.ny * geo.nz : (ax == 1 ? geo.nz : 1);
+            GlobalAxis<O> t{P.fp_in + (size_t)P_AD * N + c, P.fp_in + (size_t)(P_V1 + ax) * N + c, (size_t)N, {}};
+#pragma unroll
+            for (int q = 0; q < O; ++q) t.off[q] = (wrap(at + (q < R ? q - R : q - R + 1), n) - at) * st;
+            return t;
+          },
+          ph, sl + MAT * kThreads);
   }
 
   // ---- phase 2: the algebra of set_bd_values (bssn.cc:361-421) ----------------
@@ -815,7 +848,7 @@ __device__ __forceinline__ void stage_body(const BoxGeom& geo, const Physics& ph
   double dth[3] = {0.0, 0.0, 0.0};
   if constexpr (Z4C) {
 #pragma unroll
-    for (int d = 0; d < 3; ++d) dth[d] = S(Slots<MATTER, Z4C>::dth + d);
+    for (int d = 0; d < 3; ++d) dth[d] = S(L::dth + d);
   }
   double gm[6];
   gm[0] = g[0] + 1.0; gm[1] = g[1]; gm[2] = g[2];
@@ -852,16 +885,16 @@ __device__ __forceinline__ void stage_body(const BoxGeom& geo, const Physics& ph
   // same three of the previous substep's phi (the lagged sources); -6 phi
   // (static matter); last 5 phi and -5 phi, taken with need_H
   double phip = phi;
-  if (MATTER == kDust && stage > 1) phip = __ldcs(&P.prev[(size_t)F_PHI * N + c]) + bg.phi_FRW_prev;
-  // The parity build evaluates the batch through this thread's slots of the
-  // Christoffel symbols (free until they are formed): arguments in S_G,
-  // results in S_G + NX, the fast evaluation in a rolled loop (one copy of its
-  // code, which stays in the instruction cache), the accurate phase for the
-  // undecided ones after it; the same correctly rounded values as xexp_n.
+  if (MATTER == kDust && stage > 1) phip = __ldcs(fat(P.prev, F_PHI)) + bg.phi_FRW_prev;
+  // The parity build evaluates the batch through this thread's source slots
+  // (free until the sources are formed), in place: the fast evaluation in a
+  // rolled loop (one copy of its code, which stays in the instruction cache),
+  // the accurate phase for the undecided ones after it; the same correctly
+  // rounded values as xexp_n.
   constexpr int X6 = MATTER == kDust || MODE == kConstraints ? 1 : 0;     // 6 phi
   constexpr int XM = MATTER == kDust ? 3 : (MATTER == kStaticMatter ? 1 : 0);  // the lagged three, or -6 phi
   constexpr int X5 = 2 + X6 + XM, NX = X5 + 2;
-  static_assert(2 * NX <= 18, "the batch fits the Christoffel slots");
+  static_assert(NX <= Q_N, "the batch fits the source slots");
   double ex[NX];
   {
     double xa[NX];
@@ -879,22 +912,22 @@ __device__ __forceinline__ void stage_body(const BoxGeom& geo, const Physics& ph
     const int nx = need_H ? NX : X5;
     if constexpr (kReferenceOrder) {
 #pragma unroll
-      for (int q = 0; q < NX; ++q) S(S_G + q) = xa[q];
+      for (int q = 0; q < NX; ++q) S(SRC + q) = xa[q];
       unsigned bad = 0;
 #pragma unroll 1
       for (int q = 0; q < nx; ++q) {
         double y;
-        if (!crm::exp_fast(S(S_G + q), y)) bad |= 1u << q;
-        S(S_G + NX + q) = y;
+        if (crm::exp_fast(S(SRC + q), y)) S(SRC + q) = y;
+        else bad |= 1u << q;
       }
 #pragma unroll 1
       while (bad) {
         const int q = __ffs(bad) - 1;
         bad &= bad - 1;
-        S(S_G + NX + q) = crm::exp_full(S(S_G + q));
+        S(SRC + q) = crm::exp_full(S(SRC + q));
       }
 #pragma unroll
-      for (int q = 0; q < NX; ++q) ex[q] = S(S_G + NX + q);
+      for (int q = 0; q < NX; ++q) ex[q] = S(SRC + q);
     } else {
 #pragma unroll
       for (int q = 0; q < X5; ++q) ex[q] = xexp(xa[q]);
@@ -926,9 +959,9 @@ __device__ __forceinline__ void stage_body(const BoxGeom& geo, const Physics& ph
       const double* pv = P.prev;
       double gp[6], gip[6];
 #pragma unroll
-      for (int m = 0; m < 6; ++m) gp[m] = __ldcs(&pv[(size_t)(F_G11 + m) * N + c]);
-      const double Dp = __ldcs(&pv[(size_t)F_D * N + c]);
-      const double Sp[3] = {__ldcs(&pv[(size_t)F_S1 * N + c]), __ldcs(&pv[(size_t)F_S2 * N + c]), __ldcs(&pv[(size_t)F_S3 * N + c])};
+      for (int m = 0; m < 6; ++m) gp[m] = __ldcs(fat(pv, F_G11 + m));
+      const double Dp = __ldcs(fat(pv, F_D));
+      const double Sp[3] = {__ldcs(fat(pv, F_S1)), __ldcs(fat(pv, F_S2)), __ldcs(fat(pv, F_S3))};
       inv_metric(gp, gip);
       const DustPrim dp = dust_prim(gip, em4phip, e6phip, Dp, Sp);
       Wl = dp.W;
@@ -940,11 +973,11 @@ __device__ __forceinline__ void stage_body(const BoxGeom& geo, const Physics& ph
     double q[Q_N];
     dust_sources(Wl, detgl, gph, D, Sv, ph.lambda, q);
 #pragma unroll
-    for (int m = 0; m < Q_N; ++m) S(S_SRC + m) = q[m];
+    for (int m = 0; m < Q_N; ++m) S(SRC + m) = q[m];
     // momentum source S_m^src (dust.cc:135-146) with the current W, v
     const DustPrim cur = dust_prim(gi, em4phi, e6phi, D, Sv);
     const double e4 = e4phi;
-    rhs_m[0] = S(S_MAT + 0);
+    rhs_m[0] = S(MAT + 0);
 #pragma unroll
     for (int d = 0; d < 3; ++d) {
       const double dp = S(S_DPHI + d);
@@ -956,13 +989,13 @@ __device__ __forceinline__ void stage_body(const BoxGeom& geo, const Physics& ph
                2.0 * (cur.v[0] * cur.v[1] * (4.0 * gm[1] * dp + DG(1)) + cur.v[0] * cur.v[2] * (4.0 * gm[2] * dp + DG(2)) +
                       cur.v[1] * cur.v[2] * (4.0 * gm[4] * dp + DG(4)))) -
           cur.W * D * S(S_DA + d);
-      rhs_m[1 + d] = S(S_MAT + 1 + d) + src;
+      rhs_m[1 + d] = S(MAT + 1 + d) + src;
     }
   } else if (MATTER == kScalar) {
     // Scalar::addBSSNSource (scalar.cc:201-260) and RKEvolvePt (:85-199)
     const double sphi = C(F_SPHI), sPi = C(F_SPI);
     const double psi[3] = {C(F_SPSI1), C(F_SPSI1 + 1), C(F_SPSI1 + 2)};
-    auto SD = [&](int m, int d) { return S(S_MAT + 3 * m + d); };  // d_d of scalar field m
+    auto SD = [&](int m, int d) { return S(MAT + 3 * m + d); };  // d_d of scalar field m
     // with the shift, dt_phi = beta^i d_i phi - alpha Pi and n^mu d_mu phi =
     // (dt_phi - beta^i d_i phi) / alpha, term by term (scalar.cc:132-140, 224-229)
     double dtphi = (-alpha * sPi), nmu_num = dtphi;
@@ -978,14 +1011,14 @@ __device__ __forceinline__ void stage_body(const BoxGeom& geo, const Physics& ph
     const double dd = (gi[0] * SD(0, 0) * SD(0, 0) + gi[3] * SD(0, 1) * SD(0, 1) + gi[5] * SD(0, 2) * SD(0, 2) +
                        2.0 * (gi[1] * SD(0, 0) * SD(0, 1) + gi[2] * SD(0, 0) * SD(0, 2) + gi[4] * SD(0, 1) * SD(0, 2)));
     const double V = pot_V(ph, sphi);
-    S(S_SRC + Q_R) = 0.5 * nmu * nmu + 0.5 * em4phi * dd + V;
-    S(S_SRC + Q_S) = 3.0 / 2.0 * nmu * nmu - 0.5 * em4phi * dd - 3.0 * V;
+    S(SRC + Q_R) = 0.5 * nmu * nmu + 0.5 * em4phi * dd + V;
+    S(SRC + Q_S) = 3.0 / 2.0 * nmu * nmu - 0.5 * em4phi * dd - 3.0 * V;
 #pragma unroll
-    for (int m = 0; m < 3; ++m) S(S_SRC + Q_S1 + m) = -nmu * SD(0, m);
+    for (int m = 0; m < 3; ++m) S(SRC + Q_S1 + m) = -nmu * SD(0, m);
 #pragma unroll
     for (int I = 0; I < 3; ++I)
 #pragma unroll
-      for (int J = I; J < 3; ++J) S(S_SRC + Q_STF11 + sym(I, J)) = SD(0, I) * SD(0, J) - gm[sym(I, J)] / 3.0 * dd;
+      for (int J = I; J < 3; ++J) S(SRC + Q_STF11 + sym(I, J)) = SD(0, I) * SD(0, J) - gm[sym(I, J)] / 3.0 * dd;
     double inner = 0.0;
 #pragma unroll
     for (int X = 0; X < 3; ++X)
@@ -1025,76 +1058,154 @@ __device__ __forceinline__ void stage_body(const BoxGeom& geo, const Physics& ph
     // BSSN::clearSrc, Static::addBSSNSrc (components/static/static.cc:19-36)
     // and Lambda::addBSSNSource: the fixed density sources DIFFr only
 #pragma unroll
-    for (int m = 0; m < Q_N; ++m) S(S_SRC + m) = 0.0;
+    for (int m = 0; m < Q_N; ++m) S(SRC + m) = 0.0;
     const double phid = C(F_PHI);
     double r = 0.0;
     r += ex[2 + X6] * C(F_DIFFD) + bg.rho_FRW * xexpm1(-6.0 * phid);
     r += ph.lambda;
-    S(S_SRC + Q_R) = r;
-    S(S_SRC + Q_S) = 0.0 + -3.0 * ph.lambda;
+    S(SRC + Q_R) = r;
+    S(SRC + Q_S) = 0.0 + -3.0 * ph.lambda;
   } else {
 #pragma unroll
-    for (int m = 0; m < Q_N; ++m) S(S_SRC + m) = 0.0;
+    for (int m = 0; m < Q_N; ++m) S(SRC + m) = 0.0;
   }
 
-  // -- Christoffels (bssn.cc:577-590, bssn_macros.h:221-229) --
-  // The 18 d_I g_q are read once; the brackets d_J g_KI + d_K g_JI - d_I g_JK
-  // give the lowered symbols (half of each, which replace d_I g_q in their
-  // slots: nothing reads those afterwards) and, contracted with g^{IL}, the
-  // raised ones.
-  {
-    double dg[18];
+  // Right-hand sides are parked in slots as they are formed (the matter
+  // fields' at once, in the matter slots, which nothing reads any more), and
+  // one rolled loop below updates the registers of every field.  The BSSN
+  // fields take the slots of the lowered symbols after the Ricci tensor;
+  // theta and the shift fields follow from S_END.
+  constexpr int NM = MATTER == kDust ? 4 : (MATTER == kScalar ? 5 : 0);
+  static_assert(NFLD - F_NBSSN - NM <= L::LIVE + Q_N - S_END, "every right-hand side has a slot");
+  auto cvslot = [](int fld) {
+    return fld < F_NBSSN ? S_DG + fld : (fld < F_NBSSN + NM ? L::MAT + fld - F_NBSSN : S_END + fld - F_NBSSN - NM);
+  };
+  auto finalize = [&](int fld, double cv) { S(cvslot(fld)) = cv; };
+  if constexpr (MODE == kEvolve) {
 #pragma unroll
-    for (int q = 0; q < 18; ++q) dg[q] = S(S_DG + q);
-#pragma unroll
-    for (int J = 0; J < 3; ++J)
-#pragma unroll
-      for (int Kx = J; Kx < 3; ++Kx) {
-        const int q = sym(J, Kx);
-        double b[3];
-#pragma unroll
-        for (int I = 0; I < 3; ++I) {
-          b[I] = dg[6 * J + sym(Kx, I)] + dg[6 * Kx + sym(J, I)] - dg[6 * I + q];
-          S(S_DG + 6 * I + q) = 0.5 * b[I];
-        }
-#pragma unroll
-        for (int I = 0; I < 3; ++I) {
-          double u = gi[sym(I, 0)] * b[0];
-          u = u + gi[sym(I, 1)] * b[1];
-          u = u + gi[sym(I, 2)] * b[2];
-          S(S_G + 6 * I + q) = 0.5 * (u);
-        }
-      }
+    for (int m = 0; m < NM; ++m) finalize(F_D + m, rhs_m[m]);
   }
-  auto G = [&](int I, int qq) { return S(S_G + 6 * I + qq); };
-  auto GL = [&](int I, int qq) { return S(S_DG + 6 * I + qq); };
-  double Gd[3];
-#pragma unroll
-  for (int I = 0; I < 3; ++I)
-    Gd[I] = G(I, 0) * gi[0] + G(I, 3) * gi[3] + G(I, 5) * gi[5] + 2.0 * (G(I, 1) * gi[1] + G(I, 2) * gi[2] + G(I, 4) * gi[4]);
 
-  // -- D_i D_j phi (bssn.cc:592-602) and (D_i D_j alpha)^TF (:604-626) --
-  double dphi[3], da[3];
+  // values that wait in scratch slots: keep(n, v) stores, kept(n, v) reads
+  // back (a volatile read, so that no register holds it meanwhile)
+  auto keep = [&](int n, double v) {
+    if (n < L::NSCR) S(L::scratch(n)) = v;
+  };
+  auto kept = [&](int n, double v) -> double {
+    return n < L::NSCR ? *const_cast<const volatile double*>(&S(L::scratch(n))) : v;
+  };
+  enum : int { W_A = 0, W_G = 6, W_GD = 12, W_AA = 15 };
+
+  // -- A^ij, A_ij A^ij (calculate_Acont, bssn.cc:463-472) --
+  double A[6], Ac[6];
 #pragma unroll
-  for (int d = 0; d < 3; ++d) { dphi[d] = S(S_DPHI + d); da[d] = S(S_DA + d); }
-  double DDa[6];
-  double gld[3];
-#pragma unroll
-  for (int I = 0; I < 3; ++I) gld[I] = gi[sym(I, 0)] * dphi[0] + gi[sym(I, 1)] * dphi[1] + gi[sym(I, 2)] * dphi[2];
+  for (int q = 0; q < 6; ++q) A[q] = C(F_A11 + q);
 #pragma unroll
   for (int I = 0; I < 3; ++I)
 #pragma unroll
     for (int J = I; J < 3; ++J) {
-      const int qq = sym(I, J);
-      S(S_DDPHI + qq) = S(S_DDPHI + qq) - (G(0, qq) * dphi[0] + G(1, qq) * dphi[1] + G(2, qq) * dphi[2]);
+      double t = gi[sym(I, 0)] * gi[sym(J, 0)] * A[sym(0, 0)];
+      t = t + gi[sym(I, 1)] * gi[sym(J, 0)] * A[sym(1, 0)];
+      t = t + gi[sym(I, 2)] * gi[sym(J, 0)] * A[sym(2, 0)];
+      t = t + gi[sym(I, 0)] * gi[sym(J, 1)] * A[sym(0, 1)];
+      t = t + gi[sym(I, 1)] * gi[sym(J, 1)] * A[sym(1, 1)];
+      t = t + gi[sym(I, 2)] * gi[sym(J, 1)] * A[sym(2, 1)];
+      t = t + gi[sym(I, 0)] * gi[sym(J, 2)] * A[sym(0, 2)];
+      t = t + gi[sym(I, 1)] * gi[sym(J, 2)] * A[sym(1, 2)];
+      t = t + gi[sym(I, 2)] * gi[sym(J, 2)] * A[sym(2, 2)];
+      Ac[sym(I, J)] = t;
+    }
+  double AijAij = Ac[0] * A[0] + Ac[3] * A[3] + Ac[5] * A[5] + 2.0 * (Ac[1] * A[1] + Ac[2] * A[2] + Ac[4] * A[4]);
+
+  // -- Christoffels (bssn.cc:577-590, bssn_macros.h:221-229), D_i D_j phi
+  // (:592-602), D_i D_j alpha (:604-626) and the contractions of Gamma^I_{JK}
+  // with g^{JK} and A^{JK} --
+  // The brackets d_J g_KI + d_K g_JI - d_I g_JK of one pair (J, K) give the
+  // lowered symbols (half of each, which replace d_I g_q in their slots:
+  // nothing reads those afterwards) and, contracted with g^{IL}, the raised
+  // ones; all uses of a pair's raised symbols but Ricci term 4 follow at
+  // once, the diagonal pairs first as in the contractions' sums, so that the
+  // raised symbols take no slots.
+  double dphi[3], da[3];
+#pragma unroll
+  for (int d = 0; d < 3; ++d) { dphi[d] = S(S_DPHI + d); da[d] = S(S_DA + d); }
+  double DDa[6], gld[3];
+#pragma unroll
+  for (int I = 0; I < 3; ++I) gld[I] = gi[sym(I, 0)] * dphi[0] + gi[sym(I, 1)] * dphi[1] + gi[sym(I, 2)] * dphi[2];
+  double Gd[3], so[3];
+  double gv[3], gs[3];  // constraint mode: the Christoffel constraint and its scale
+  {
+    double dg[18];
+#pragma unroll
+    for (int q = 0; q < 18; ++q) dg[q] = S(S_DG + q);
+    double Gx[3], sx[3];  // the sums over the mixed pairs
+    constexpr int pair[6] = {0, 3, 5, 1, 2, 4};
+#pragma unroll
+    for (int n = 0; n < 6; ++n) {
+      const int q = pair[n];
+      const int J = q < 3 ? 0 : (q < 5 ? 1 : 2), Kx = q < 3 ? q : (q < 5 ? q - 2 : 2);  // sym(J, Kx) = q
+      double b[3], Gq[3];
+#pragma unroll
+      for (int I = 0; I < 3; ++I) {
+        b[I] = dg[6 * J + sym(Kx, I)] + dg[6 * Kx + sym(J, I)] - dg[6 * I + q];
+        S(S_DG + 6 * I + q) = 0.5 * b[I];
+      }
+#pragma unroll
+      for (int I = 0; I < 3; ++I) {
+        double u = gi[sym(I, 0)] * b[0];
+        u = u + gi[sym(I, 1)] * b[1];
+        u = u + gi[sym(I, 2)] * b[2];
+        Gq[I] = 0.5 * (u);
+        const double x = Gq[I] * gi[q], y = Gq[I] * Ac[q];
+        if (n < 3) {
+          Gd[I] = n == 0 ? x : Gd[I] + x;
+          so[I] = n == 0 ? y : so[I] + y;
+          if constexpr (MODE == kConstraints) {
+            gv[I] = (n == 0 ? C(F_GAM1 + I) : gv[I]) - x;
+            gs[I] = n == 0 ? x : gs[I] - x;
+          }
+        } else {
+          Gx[I] = n == 3 ? x : Gx[I] + x;
+          sx[I] = n == 3 ? y : sx[I] + y;
+        }
+      }
+      S(S_DDPHI + q) = S(S_DDPHI + q) - (Gq[0] * dphi[0] + Gq[1] * dphi[1] + Gq[2] * dphi[2]);
       double t = 0.0;
 #pragma unroll
-      for (int L = 0; L < 3; ++L) {
-        const double u = G(L, qq) + 2.0 * ((L == I ? 1.0 : 0.0) * dphi[J] + (L == J ? 1.0 : 0.0) * dphi[I] - gm[qq] * gld[L]);
-        t = L == 0 ? u * da[L] : t + u * da[L];
+      for (int l = 0; l < 3; ++l) {
+        const double u = Gq[l] + 2.0 * ((l == J ? 1.0 : 0.0) * dphi[Kx] + (l == Kx ? 1.0 : 0.0) * dphi[J] - gm[q] * gld[l]);
+        t = l == 0 ? u * da[l] : t + u * da[l];
       }
-      DDa[qq] = S(S_DDA + qq) - (t);
+      DDa[q] = S(S_DDA + q) - (t);
     }
+#pragma unroll
+    for (int I = 0; I < 3; ++I) {
+      if constexpr (MODE == kConstraints) {  // BSSN_GI_CALC / BSSN_GI_SCALE (bssn_macros.h:530-536)
+        gv[I] = gv[I] - 2.0 * Gx[I];
+        gs[I] = fabs(C(F_GAM1 + I)) + fabs(gs[I] - 2.0 * Gx[I]);
+      }
+      Gd[I] = Gd[I] + 2.0 * Gx[I];
+      so[I] = (so[I] + 2.0 * sx[I]) + 6.0 * (Ac[sym(I, 0)] * dphi[0] + Ac[sym(I, 1)] * dphi[1] + Ac[sym(I, 2)] * dphi[2]);
+    }
+  }
+  auto GL = [&](int I, int qq) { return S(S_DG + 6 * I + qq); };
+  // ev_GammaI (bssn.cc:762-764, BSSN_DT_GAMMAI_NOSHIFT bssn_macros.h:342-361)
+  // without the shift's terms, into the slots of d_I K
+  if constexpr (MODE == kEvolve) {
+    const double sq[3] = {S(SRC + Q_S1), S(SRC + Q_S2), S(SRC + Q_S3)};
+    const double dK[3] = {S(S_DK + 0), S(S_DK + 1), S(S_DK + 2)};
+#pragma unroll
+    for (int I = 0; I < 3; ++I)
+      S(S_DK + I) =
+          (-2.0 * (Ac[sym(I, 0)] * da[0] + Ac[sym(I, 1)] * da[1] + Ac[sym(I, 2)] * da[2]) +
+           2.0 * alpha *
+               (+so[I] -
+                (1.0 / 3.0) * (2.0 * (gi[sym(I, 0)] * dK[0] + gi[sym(I, 1)] * dK[1] + gi[sym(I, 2)] * dK[2]) +
+                               gi[sym(I, 0)] * dth[0] + gi[sym(I, 1)] * dth[1] + gi[sym(I, 2)] * dth[2]) -
+                2.0 * alpha * k1 * (C(F_GAM1 + I) - Gd[I]) -
+                8.0 * kPi * (gi[sym(I, 0)] * sq[0] + gi[sym(I, 1)] * sq[1] + gi[sym(I, 2)] * sq[2])));
+  }
+  // (D_i D_j alpha)^TF (bssn.cc:604-626)
   double DDaTR = gi[0] * DDa[0] + gi[3] * DDa[3] + gi[5] * DDa[5] + 2.0 * (gi[1] * DDa[1] + gi[2] * DDa[2] + gi[4] * DDa[4]);
 #pragma unroll
   for (int m = 0; m < 6; ++m) S(S_DDA + m) = DDa[m] - (1.0 / 3.0) * gm[m] * DDaTR;
@@ -1119,19 +1230,46 @@ __device__ __forceinline__ void stage_body(const BoxGeom& geo, const Physics& ph
   // order: the FMA build uses it.  The parity build (kReferenceOrder) sums
   // the reference's terms in the reference's order, so that its rounding is
   // the reference's.
-  double t4[6] = {0.0, 0.0, 0.0, 0.0, 0.0, 0.0};
-  if constexpr (kReferenceOrder) {
-    // the parity build: the reference's 27 terms per component, summed over
-    // (K, L, M) with M fastest, each term formed as the macro forms it; the
-    // six components advance together, so the symbols of one K are loaded
-    // once for all of them.  K is a rolled loop: its body (54 terms) stays
-    // in the instruction cache for the second and third pass, where the
-    // unrolled 162 terms did not (the slot addresses take K at run time; the
-    // sum starts from +0, which changes no value)
-#pragma unroll 1
-    for (int Kx = 0; Kx < 3; ++Kx)
 #pragma unroll
-      for (int L = 0; L < 3; ++L)
+  for (int q = 0; q < 6; ++q) {
+    keep(W_A + q, A[q]);
+    keep(W_G + q, g[q]);
+    if (q < 3) keep(W_GD + q, Gd[q]);
+  }
+  keep(W_AA, AijAij);
+  double t4[6] = {0.0, 0.0, 0.0, 0.0, 0.0, 0.0};
+  // one K at a time in a rolled loop, whose body stays in the instruction
+  // cache; the raised symbols of that K again from the lowered ones (the
+  // halves and doublings of the two forms are exact, so the values are those
+  // formed above)
+#pragma unroll 1
+  for (int Kx = 0; Kx < 3; ++Kx) {
+    double Gk[6];  // Gamma^K_q
+    {
+      const double r0 = Kx == 0 ? gi[0] : (Kx == 1 ? gi[1] : gi[2]), r1 = Kx == 0 ? gi[1] : (Kx == 1 ? gi[3] : gi[4]),
+                   r2 = Kx == 0 ? gi[2] : (Kx == 1 ? gi[4] : gi[5]);
+#pragma unroll
+      for (int q = 0; q < 6; ++q) {
+        double u = r0 * GL(0, q);
+        u = u + r1 * GL(1, q);
+        Gk[q] = u + r2 * GL(2, q);
+      }
+    }
+    const int kq[3] = {Kx, Kx == 0 ? 1 : Kx + 2, Kx == 0 ? 2 : Kx + 3};  // sym(Kx, M)
+    double Gj[3][3], Gl[6];  // Gamma_{J, K M}, Gamma_{K, q}
+#pragma unroll
+    for (int J = 0; J < 3; ++J)
+#pragma unroll
+      for (int M = 0; M < 3; ++M) Gj[J][M] = GL(J, kq[M]);
+#pragma unroll
+    for (int q = 0; q < 6; ++q) Gl[q] = GL(Kx, q);
+    if constexpr (kReferenceOrder) {
+      // the parity build: the reference's 27 terms per component, summed over
+      // (K, L, M) with M fastest, each term formed as the macro forms it, the
+      // six components advancing together (the sum starts from +0, which
+      // changes no value)
+#pragma unroll
+      for (int l = 0; l < 3; ++l)
 #pragma unroll
         for (int M = 0; M < 3; ++M)
 #pragma unroll
@@ -1139,71 +1277,58 @@ __device__ __forceinline__ void stage_body(const BoxGeom& geo, const Physics& ph
 #pragma unroll
             for (int J = I; J < 3; ++J) {
               const double u =
-                  gi[sym(L, M)] * (G(Kx, sym(L, I)) * GL(J, sym(Kx, M)) + G(Kx, sym(L, J)) * GL(I, sym(Kx, M)) +
-                                   0.5 * (G(Kx, sym(I, M)) * GL(Kx, sym(L, J)) + G(Kx, sym(J, M)) * GL(Kx, sym(L, I))));
+                  gi[sym(l, M)] * (Gk[sym(l, I)] * Gj[J][M] + Gk[sym(l, J)] * Gj[I][M] +
+                                   0.5 * (Gk[sym(I, M)] * Gl[sym(l, J)] + Gk[sym(J, M)] * Gl[sym(l, I)]));
               t4[sym(I, J)] = t4[sym(I, J)] + u;
             }
-  } else {
+    } else {
+      double Hm[3][3];  // H^K_{MX} = sum_L g^{LM} G^K_{LX}
 #pragma unroll
-  for (int Kx = 0; Kx < 3; ++Kx) {
-    double Hm[3][3];  // H^K_{MX} = sum_L g^{LM} G^K_{LX}
+      for (int M = 0; M < 3; ++M)
 #pragma unroll
-    for (int M = 0; M < 3; ++M)
+        for (int X = 0; X < 3; ++X)
+          Hm[M][X] = gi[sym(0, M)] * Gk[sym(0, X)] + gi[sym(1, M)] * Gk[sym(1, X)] + gi[sym(2, M)] * Gk[sym(2, X)];
 #pragma unroll
-      for (int X = 0; X < 3; ++X)
-        Hm[M][X] = gi[sym(0, M)] * G(Kx, sym(0, X)) + gi[sym(1, M)] * G(Kx, sym(1, X)) + gi[sym(2, M)] * G(Kx, sym(2, X));
+      for (int I = 0; I < 3; ++I)
 #pragma unroll
-    for (int I = 0; I < 3; ++I)
+        for (int J = I; J < 3; ++J) {
+          double u = 0.0, w = 0.0;
 #pragma unroll
-      for (int J = I; J < 3; ++J) {
-        double u = 0.0, w = 0.0;
-#pragma unroll
-        for (int M = 0; M < 3; ++M) {
-          u = u + (Hm[M][I] * GL(J, sym(Kx, M)) + Hm[M][J] * GL(I, sym(Kx, M)));
-          w = w + (Hm[M][I] * GL(Kx, sym(M, J)) + Hm[M][J] * GL(Kx, sym(M, I)));
+          for (int M = 0; M < 3; ++M) {
+            u = u + (Hm[M][I] * Gj[J][M] + Hm[M][J] * Gj[I][M]);
+            w = w + (Hm[M][I] * Gl[sym(M, J)] + Hm[M][J] * Gl[sym(M, I)]);
+          }
+          t4[sym(I, J)] = t4[sym(I, J)] + (u + 0.5 * w);
         }
-        t4[sym(I, J)] = t4[sym(I, J)] + (u + 0.5 * w);
-      }
+    }
   }
+#pragma unroll
+  for (int q = 0; q < 6; ++q) {
+    g[q] = kept(W_G + q, g[q]);
+    gm[q] = (q == 0 || q == 3 || q == 5) ? g[q] + 1.0 : g[q];
+    if (q < 3) {
+      Gd[q] = kept(W_GD + q, Gd[q]);
+      dphi[q] = *const_cast<const volatile double*>(&S(S_DPHI + q));
+    }
   }
 #pragma unroll
   for (int I = 0; I < 3; ++I)
 #pragma unroll
     for (int J = I; J < 3; ++J) {
       const int ij = sym(I, J);
-      auto dGam = [&](int Jx, int Kx) { return S(S_DGAM + 3 * Kx + Jx); };
-      const double t2a = gm[sym(0, I)] * dGam(J, 0) + gm[sym(1, I)] * dGam(J, 1) + gm[sym(2, I)] * dGam(J, 2);
-      const double t2b = gm[sym(0, J)] * dGam(I, 0) + gm[sym(1, J)] * dGam(I, 1) + gm[sym(2, J)] * dGam(I, 2);
       const double t3a = Gd[0] * GL(I, sym(J, 0)) + Gd[1] * GL(I, sym(J, 1)) + Gd[2] * GL(I, sym(J, 2));
       const double t3b = Gd[0] * GL(J, sym(I, 0)) + Gd[1] * GL(J, sym(I, 1)) + Gd[2] * GL(J, sym(I, 2));
-      const double U = (-0.5 * (S(S_T1 + ij)) + 0.5 * (t2a + t2b) + 0.5 * (t3a + t3b) + t4[ij]);
+      const double U = (S(S_T1 + ij) + 0.5 * (t3a + t3b) + t4[ij]);  // terms 1 and 2 were joined in phase 1
       S(S_T1 + ij) = U - 2.0 * (DDphi(ij) - 2.0 * dphi[I] * dphi[J] + gm[ij] * (expression));
     }
   auto Ric = [&](int qq) { return S(S_T1 + qq); };  // full Ricci R_ij (bssn.cc:650-655)
   const double ricci = em4phi * (Ric(0) * gi[0] + Ric(3) * gi[3] + Ric(5) * gi[5] +
                                  2.0 * (Ric(1) * gi[1] + Ric(2) * gi[2] + Ric(4) * gi[4]));
 
-  // -- A^ij, A_ij A^ij (calculate_Acont, bssn.cc:463-472) --
-  double A[6], Ac[6];
 #pragma unroll
-  for (int q = 0; q < 6; ++q) A[q] = C(F_A11 + q);
-#pragma unroll
-  for (int I = 0; I < 3; ++I)
-#pragma unroll
-    for (int J = I; J < 3; ++J) {
-      double t = gi[sym(I, 0)] * gi[sym(J, 0)] * A[sym(0, 0)];
-      t = t + gi[sym(I, 1)] * gi[sym(J, 0)] * A[sym(1, 0)];
-      t = t + gi[sym(I, 2)] * gi[sym(J, 0)] * A[sym(2, 0)];
-      t = t + gi[sym(I, 0)] * gi[sym(J, 1)] * A[sym(0, 1)];
-      t = t + gi[sym(I, 1)] * gi[sym(J, 1)] * A[sym(1, 1)];
-      t = t + gi[sym(I, 2)] * gi[sym(J, 1)] * A[sym(2, 1)];
-      t = t + gi[sym(I, 0)] * gi[sym(J, 2)] * A[sym(0, 2)];
-      t = t + gi[sym(I, 1)] * gi[sym(J, 2)] * A[sym(1, 2)];
-      t = t + gi[sym(I, 2)] * gi[sym(J, 2)] * A[sym(2, 2)];
-      Ac[sym(I, J)] = t;
-    }
-  const double AijAij = Ac[0] * A[0] + Ac[3] * A[3] + Ac[5] * A[5] + 2.0 * (Ac[1] * A[1] + Ac[2] * A[2] + Ac[4] * A[4]);
-  const double r = S(S_SRC + Q_R) + bg.rho_FRW;
+  for (int q = 0; q < 6; ++q) A[q] = kept(W_A + q, A[q]);
+  AijAij = kept(W_AA, AijAij);
+  const double r = S(SRC + Q_R) + bg.rho_FRW;
   // Hamiltonian constraint, bssn.cc:1073-1084 (theta = 0)
   const double H = need_H ? -e5phi / 8.0 * (ricci + 2.0 / 3.0 * ((K + 2.0 * theta) * (K + 2.0 * theta)) - AijAij - 16.0 * kPi * r) : 0.0;
 
@@ -1228,20 +1353,13 @@ __device__ __forceinline__ void stage_body(const BoxGeom& geo, const Physics& ph
             const double u = gi[sym(X, d)] * A[sym(X, I)] * dphi[d];
             t6 = (d == 0 && X == 0) ? u : t6 + u;
           }
-        double tD = 0.0;
-#pragma unroll
-        for (int X = 0; X < 3; ++X)
-#pragma unroll
-          for (int d = 0; d < 3; ++d) {
-            const double u = gi[sym(X, d)] * S(SlotsC<MATTER, Z4C>::dA + 3 * sym(X, I) + d);
-            tD = (X == 0 && d == 0) ? u : tD + u;
-          }
+        double tD = S(L::dA + I);  // g^{Xd} d_d A_{XI}, from phase 1
         tD = tD - Gd[0] * A[sym(0, I)] - Gd[1] * A[sym(1, I)] - Gd[2] * A[sym(2, I)];
 #pragma unroll
         for (int X = 0; X < 3; ++X)
 #pragma unroll
           for (int Y = 0; Y < 3; ++Y) tD = tD - GL(Y, sym(X, I)) * Ac[sym(Y, X)];
-        const double sI = S(S_SRC + Q_S1 + I);
+        const double sI = S(SRC + Q_S1 + I);
         mv[I] = e6 * (-2.0 / 3.0 * S(S_DK + I) - 8 * kPi * (sI) - 2.0 / 3.0 * 2.0 * dth[I] + 6.0 * (t6) + (tD));
         ms[I] = e6 * (fabs(2.0 / 3.0 * S(S_DK + I)) + fabs(8 * kPi * (sI)) + fabs(2.0 / 3.0 * 2.0 * dth[I]) +
                       6.0 * fabs(t6) + fabs(tD));
@@ -1249,19 +1367,9 @@ __device__ __forceinline__ void stage_body(const BoxGeom& geo, const Physics& ph
       v[1] = sqrt(mv[0] * mv[0] + mv[1] * mv[1] + mv[2] * mv[2]);
       sc[1] = sqrt(ms[0] * ms[0] + ms[1] * ms[1] + ms[2] * ms[2]);
     }
-    {  // christoffel constraint, BSSN_GI_CALC / BSSN_GI_SCALE (bssn_macros.h:530-536)
-      double gv[3], gs[3];
-#pragma unroll
-      for (int I = 0; I < 3; ++I) {
-        const double Gam = C(F_GAM1 + I);
-        gv[I] = Gam - gi[0] * G(I, 0) - gi[3] * G(I, 3) - gi[5] * G(I, 5) -
-                2.0 * (gi[1] * G(I, 1) + gi[2] * G(I, 2) + gi[4] * G(I, 4));
-        gs[I] = fabs(Gam) + fabs(gi[0] * G(I, 0) - gi[3] * G(I, 3) - gi[5] * G(I, 5) -
-                                 2.0 * (gi[1] * G(I, 1) + gi[2] * G(I, 2) + gi[4] * G(I, 4)));
-      }
-      v[2] = sqrt(gv[0] * gv[0] + gv[1] * gv[1] + gv[2] * gv[2]);
-      sc[2] = sqrt(gs[0] * gs[0] + gs[1] * gs[1] + gs[2] * gs[2]);
-    }
+    // christoffel constraint
+    v[2] = sqrt(gv[0] * gv[0] + gv[1] * gv[1] + gv[2] * gv[2]);
+    sc[2] = sqrt(gs[0] * gs[0] + gs[1] * gs[1] + gs[2] * gs[2]);
     // AijTFConstraintCalc / Scale (bssn.cc:1182-1192)
     v[3] = gi[0] * A[0] + gi[3] * A[3] + gi[5] * A[5] + 2.0 * (gi[1] * A[1] + gi[2] * A[2] + gi[4] * A[4]);
     sc[3] = fabs(gi[0] * A[0]) + fabs(gi[3] * A[3]) + fabs(gi[5] * A[5]) +
@@ -1291,7 +1399,7 @@ __device__ __forceinline__ void stage_body(const BoxGeom& geo, const Physics& ph
     if (live) {
       // ricci_a (bssn.cc:663) and DIFFr_a at this point, for io_bssn_dump_statistics
       P.cvals[(size_t)10 * N + c] = ricci;
-      P.cvals[(size_t)11 * N + c] = S(S_SRC + Q_R);
+      P.cvals[(size_t)11 * N + c] = S(SRC + Q_R);
     }
     q[15] = live ? v[0] * v[0] * dx * dx * dx : 0.0;
     q[16] = live ? v[1] * v[1] * dx * dx * dx : 0.0;
@@ -1318,14 +1426,6 @@ __device__ __forceinline__ void stage_body(const BoxGeom& geo, const Physics& ph
     }
   }
   auto ko = [&](int fld) -> double { return ko_on ? S(S_DG + fld) : 0.0; };
-  // Each right-hand side is parked in a slot free in the epilogue (the
-  // lowered Christoffels for the 18 BSSN fields, after the field's
-  // dissipation value there has been read; d_J Gamma^K and D_i D_j phi for the
-  // rest), and one rolled loop below updates the registers of every field.
-  static_assert(NFLD <= F_NBSSN + 9 + 6, "every right-hand side has a slot");
-  auto cvslot = [](int fld) { return fld < F_NBSSN ? S_DG + fld : (fld < F_NBSSN + 9 ? S_DGAM + fld - F_NBSSN : S_DDPHI + fld - F_NBSSN - 9); };
-  auto finalize = [&](int fld, double cv) { S(cvslot(fld)) = cv; };
-
   // ev_DIFFgammaIJ (bssn.cc:748-753, BSSN_DT_DIFFGAMMAIJ bssn_macros.h:292-307)
 #pragma unroll
   for (int I = 0; I < 3; ++I)
@@ -1363,7 +1463,7 @@ __device__ __forceinline__ void stage_body(const BoxGeom& geo, const Physics& ph
           aa = (X == 0 && Y == 0) ? u : aa + u;
         }
       const double RTF = Ric(qq) - (1.0 / 3.0) * e4phi * gm[qq] * ricci;
-      double dtA = (em4phi * (alpha * (RTF - 8.0 * kPi * S(S_SRC + Q_STF11 + qq)) - S(S_DDA + qq)) +
+      double dtA = (em4phi * (alpha * (RTF - 8.0 * kPi * S(SRC + Q_STF11 + qq)) - S(S_DDA + qq)) +
                     alpha * (((K + 2.0 * theta) * A[qq]) - 2.0 * (aa)));
       if constexpr (SHIFT) {  // BSSN_DT_AIJ with the shift (bssn_macros.h:319-332)
 #pragma unroll
@@ -1378,21 +1478,10 @@ __device__ __forceinline__ void stage_body(const BoxGeom& geo, const Physics& ph
       if constexpr (SHIFT) rhsA[qq] = evA;
       finalize(F_A11 + qq, evA);
     }
-  // ev_GammaI (bssn.cc:762-764, BSSN_DT_GAMMAI_NOSHIFT bssn_macros.h:342-361)
-  const double sq[3] = {S(S_SRC + Q_S1), S(S_SRC + Q_S2), S(S_SRC + Q_S3)};
+  // ev_GammaI: the part formed above and the shift's
 #pragma unroll
   for (int I = 0; I < 3; ++I) {
-    auto Gs = [&](int qq) { return S(S_G + 6 * I + qq); };
-    const double so = (Gs(0) * Ac[0] + Gs(3) * Ac[3] + Gs(5) * Ac[5] + 2.0 * (Gs(1) * Ac[1] + Gs(2) * Ac[2] + Gs(4) * Ac[4]) +
-                       6.0 * (Ac[sym(I, 0)] * dphi[0] + Ac[sym(I, 1)] * dphi[1] + Ac[sym(I, 2)] * dphi[2]));
-    const double ns =
-        (-2.0 * (Ac[sym(I, 0)] * da[0] + Ac[sym(I, 1)] * da[1] + Ac[sym(I, 2)] * da[2]) +
-         2.0 * alpha *
-             (+so -
-              (1.0 / 3.0) * (2.0 * (gi[sym(I, 0)] * S(S_DK + 0) + gi[sym(I, 1)] * S(S_DK + 1) + gi[sym(I, 2)] * S(S_DK + 2)) +
-                             gi[sym(I, 0)] * dth[0] + gi[sym(I, 1)] * dth[1] + gi[sym(I, 2)] * dth[2]) -
-              2.0 * alpha * k1 * (C(F_GAM1 + I) - Gd[I]) -
-              8.0 * kPi * (gi[sym(I, 0)] * sq[0] + gi[sym(I, 1)] * sq[1] + gi[sym(I, 2)] * sq[2])));
+    const double ns = S(S_DK + I);
     if constexpr (SHIFT) {
       // BSSN_DT_GAMMAI_SHIFT (bssn_macros.h:363-382), term by term
       double sh = up(F_GAM1 + I, 0);
@@ -1424,7 +1513,7 @@ __device__ __forceinline__ void stage_body(const BoxGeom& geo, const Physics& ph
   // ev_DIFFK (bssn.cc:766-795)
   {
     double v = (-DDaTR + alpha * (1.0 / 3.0 * (Kd + 2.0 * theta) * (Kd + 2.0 * theta + 2.0 * bg.K_FRW) + AijAij) +
-                4.0 * kPi * alpha * (S(S_SRC + Q_R) + S(S_SRC + Q_S)) + 4.0 * kPi * alphad * (bg.rho_FRW + bg.S_FRW));
+                4.0 * kPi * alpha * (S(SRC + Q_R) + S(SRC + Q_S)) + 4.0 * kPi * alphad * (bg.rho_FRW + bg.S_FRW));
     if constexpr (SHIFT) {
 #pragma unroll
       for (int d = 0; d < 3; ++d) v = v + up(F_K, d);
@@ -1512,13 +1601,7 @@ __device__ __forceinline__ void stage_body(const BoxGeom& geo, const Physics& ph
       finalize(F_EXPN, v - alpha * K / 3.0);
     }
   }
-  if (MATTER == kDust) {
-#pragma unroll
-    for (int m = 0; m < 4; ++m) finalize(F_D + m, rhs_m[m]);
-  } else if (MATTER == kScalar) {
-#pragma unroll
-    for (int m = 0; m < 5; ++m) finalize(F_SPHI + m, rhs_m[m]);
-  } else if (MATTER == kStaticMatter) {
+  if (MATTER == kStaticMatter) {
     // the fixed density is no register of the reference: every output keeps it
     const double pv = __ldcs(&P.p[(size_t)F_DIFFD * N + c]);
     __stcs(&P.out[(size_t)F_DIFFD * N + c], pv);
@@ -1527,8 +1610,8 @@ __device__ __forceinline__ void stage_body(const BoxGeom& geo, const Physics& ph
   }
 
   // RK4Register::K{n}Finalize (RK4Register.h:180-230) of every field, one
-  // rolled loop (one copy of the code) with the next field's registers
-  // loaded while this one is updated; the substep's divisors chosen once:
+  // rolled loop, the registers of eight fields loaded at once (in flight
+  // together); the substep's divisors chosen once:
   // f = f + dt cv / 6 (substep 1, from f = 0), / 3 (2, 3); a = p + dt cv / 2
   // (1, 2), / 1 (3); p = f + (dt cv / 6 + p) (4).  0 + x = x, so the values
   // are those of the four separate forms.  The new values replace the
@@ -1539,36 +1622,54 @@ __device__ __forceinline__ void stage_body(const BoxGeom& geo, const Physics& ph
     const bool by6 = stage == 1 || stage == 4;
     const Divisor by{by6 ? 6.0 : 3.0, by6 ? 1.0 / 6.0 : 1.0 / 3.0, by6 ? kSixthLo : 2.0 * kSixthLo};
     const double ahead = stage == 3 ? 1.0 : 0.5;
-    auto skip = [](int fld) { return MATTER == kStaticMatter && fld == F_DIFFD; };
-    double pv = __ldcs(&P.p[c]);
-    double fv = stage == 1 ? 0.0 : __ldcs(&P.f[c]);
+    auto update = [&](auto last) {
+      constexpr bool kLast = decltype(last)::value;
+      constexpr int CH = 8;
 #pragma unroll 1
-    for (int fld = 0; fld < NFLD; ++fld) {
-      const double pcur = pv, fcur = fv;
-      if (fld + 1 < NFLD) {
-        pv = __ldcs(&P.p[(size_t)(fld + 1) * N + c]);
-        fv = stage == 1 ? 0.0 : __ldcs(&P.f[(size_t)(fld + 1) * N + c]);
+      for (int f0 = 0; f0 < NFLD; f0 += CH) {
+        double pv[CH], fv[CH], t[CH], d[CH];
+        bool odd = false;
+#pragma unroll
+        for (int q = 0; q < CH; ++q) {
+          if (f0 + q >= NFLD) continue;
+          pv[q] = __ldcs(fat(P.p, f0 + q));
+          fv[q] = !kLast && stage == 1 ? 0.0 : __ldcs(fat(P.f, f0 + q));
+        }
+#pragma unroll
+        for (int q = 0; q < CH; ++q) {
+          if (f0 + q >= NFLD) continue;
+          t[q] = dt * S(cvslot(f0 + q));
+          d[q] = by(t[q]);
+          odd |= DivRange::outside(t[q]);
+        }
+        if (odd) {  // a zero (whose sign stays), or outside the divisor's range
+#pragma unroll
+          for (int q = 0; q < CH; ++q) {
+            if (f0 + q >= NFLD) continue;
+            if (DivRange::outside(t[q])) d[q] = t[q] == 0.0 ? t[q] : t[q] / by.d;
+          }
+        }
+#pragma unroll
+        for (int q = 0; q < CH; ++q) {
+          const int fld = f0 + q;
+          if (fld >= NFLD || (MATTER == kStaticMatter && fld == F_DIFFD)) continue;
+          double o;
+          if constexpr (kLast) {
+            o = fv[q] + (d[q] + pv[q]);
+            // the new state is also the next step's first input, except gamma
+            // and A, which are renormalised below
+            if (!(renorm && fld < F_K && fld != F_PHI)) __stcs(fat(P.norm, fld), o);
+          } else {
+            __stcs(fat(P.f, fld), fv[q] + d[q]);
+            o = pv[q] + t[q] * ahead;
+          }
+          __stcs(fat(P.out, fld), o);
+          S(cvslot(fld)) = o;
+        }
       }
-      if (skip(fld)) continue;
-      const double t = dt * S(cvslot(fld));
-      DivRange rg;
-      rg.numerator(t);
-      double q = by(t);
-      if (!rg.ok()) q = t / by.d;
-      if (t == 0.0) q = t;  // the zero's own sign
-      double o;
-      if (stage == 4) {
-        o = fcur + (q + pcur);
-      } else {
-        __stcs(&P.f[(size_t)fld * N + c], fcur + q);
-        o = pcur + t * ahead;
-      }
-      __stcs(&P.out[(size_t)fld * N + c], o);
-      // at the last substep the new state is also the next step's first
-      // input, except gamma and A, which are renormalised below
-      if (stage == 4 && !(renorm && fld < F_K && fld != F_PHI)) __stcs(&P.norm[(size_t)fld * N + c], o);
-      S(cvslot(fld)) = o;
-    }
+    };
+    if (stage == 4) update(std::true_type());
+    else update(std::false_type());
   }
 #pragma unroll
   for (int f = 0; f < NFLD; ++f) outv[f] = S(cvslot(f));
@@ -1593,8 +1694,8 @@ __device__ __forceinline__ void stage_body(const BoxGeom& geo, const Physics& ph
       for (int m = 0; m < 6; ++m) {
         outv[F_G11 + m] = gn[m];
         outv[F_A11 + m] = An[m];
-        __stcs(&P.norm[(size_t)(F_G11 + m) * N + c], gn[m]);
-        __stcs(&P.norm[(size_t)(F_A11 + m) * N + c], An[m]);
+        __stcs(fat(P.norm, F_G11 + m), gn[m]);
+        __stcs(fat(P.norm, F_A11 + m), An[m]);
       }
     }
   }
@@ -1614,19 +1715,20 @@ __device__ __forceinline__ void stage_body(const BoxGeom& geo, const Physics& ph
     const DustPrim dp = dust_prim(gio, eo[0], eo[1], outv[F_D], So);
     const double alo = outv[F_ALPHA] + 1.0;
     double* fo = P.fp_out;
-    __stcs(&fo[(size_t)P_AD * N + c], alo * outv[F_D]);
+    __stcs(fat(fo, P_AD), alo * outv[F_D]);
 #pragma unroll
-    for (int m = 0; m < 3; ++m) __stcs(&fo[(size_t)(P_AS1 + m) * N + c], alo * So[m]);
+    for (int m = 0; m < 3; ++m) __stcs(fat(fo, P_AS1 + m), alo * So[m]);
 #pragma unroll
-    for (int m = 0; m < 3; ++m) __stcs(&fo[(size_t)(P_V1 + m) * N + c], dp.v[m]);
+    for (int m = 0; m < 3; ++m) __stcs(fat(fo, P_V1 + m), dp.v[m]);
   }
 }
 
-// the two TMA barriers of a CTA: initialised once, before any copy
+// the TMA barriers of a CTA: initialised once, before any copy
 __device__ __forceinline__ void init_tile_barriers(uint64_t* bar, bool use) {
   if (use && threadIdx.x == 0 && threadIdx.y == 0 && threadIdx.z == 0) {
     tma::bar_init(bar, 1);
     tma::bar_init(bar + 1, 1);
+    tma::bar_init(bar + 2, 1);
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
   __syncthreads();
@@ -1635,10 +1737,10 @@ __device__ __forceinline__ void init_tile_barriers(uint64_t* bar, bool use) {
 // One box: one CTA per brick.  tmap: the TMA map of this substep's input
 // (use_tma = 0: every tile is copied by the threads).
 template <int O, int MATTER, int MODE, bool KO = false, bool Z4C = false, bool SHIFT = false>
-__global__ void __launch_bounds__(kThreads, 2)
+__global__ void __launch_bounds__(kThreads, 1)
 stage_kernel(BoxGeom geo, Physics ph, StageBg bg, StagePtrs P, int stage, const __grid_constant__ CUtensorMap tmap,
              int use_tma, const __grid_constant__ FluxMaps fmaps, int use_fmaps) {
-  __shared__ __align__(8) uint64_t bar[2];
+  __shared__ __align__(8) uint64_t bar[3];
   init_tile_barriers(bar, use_tma != 0);
   unsigned phase = 0;
   bool tma_ok = true;
@@ -1654,14 +1756,14 @@ stage_kernel(BoxGeom geo, Physics ph, StageBg bg, StagePtrs P, int stage, const 
 // items blockIdx.x, blockIdx.x + gridDim.x, ... (a persistent launch when the
 // grid is smaller than the list).
 template <int O, int MATTER>
-__global__ void __launch_bounds__(kThreads, 2)
+__global__ void __launch_bounds__(kThreads, 1)
 stage_group_kernel(const GroupBox* __restrict__ boxes, GroupBg gb, int stage) {
   __shared__ GroupBox sb;
   __shared__ StagePtrs sp;
   __shared__ StageBg sbg;
   __shared__ const CUtensorMap* stm;
   __shared__ const FluxMaps* sfm;
-  __shared__ __align__(8) uint64_t bar[2];
+  __shared__ __align__(8) uint64_t bar[3];
   const bool lead = threadIdx.x == 0 && threadIdx.y == 0 && threadIdx.z == 0;
   init_tile_barriers(bar, true);
   unsigned phase = 0;

@@ -81,7 +81,7 @@ cudaError_t go_stage(const BoxDev& b, const StageBg& bg, int stage, cudaStream_t
   const CUtensorMap* fsrc = (stage == 1 || stage == 3) ? b.fmap0 : b.fmap1;
   for (int a = 0; a < 3; ++a) fm.m[a] = fsrc[a];
   constexpr bool Z = kZ4cUnit;
-  constexpr size_t smem = stage_smem<O, M, kEvolve, Z>();
+  constexpr size_t smem = Layout<O, M, kEvolve, Z, kShiftUnit>::kBytes;
   if constexpr (kShiftUnit) {
     // one instantiation per order and matter; the dissipation is switched at run time
     static bool configured_shift = false;
@@ -146,7 +146,7 @@ cudaError_t go_constraints(const BoxDev& b, const StageBg& bg, double* cvals, do
   P.cpart = cpart;
   BoxGeom geo{b.nx, b.ny, b.nz, b.pts, b.xg / kBX};
   constexpr bool Z = kZ4cUnit;
-  constexpr size_t smem = stage_smem<O, M, kConstraints, Z>();
+  constexpr size_t smem = Layout<O, M, kConstraints, Z>::kBytes;
   static bool configured = false;
   if (!configured) {
     cudaError_t e = cudaFuncSetAttribute(stage_kernel<O, M, kConstraints, false, Z>,
@@ -174,7 +174,7 @@ cudaError_t go_constraints_m(const BoxDev& b, const StageBg& bg, double* cvals, 
 #if !CG_AUX_UNIT
 template <int O, int M>
 cudaError_t go_group(const GroupBox* table, const GroupBg& gb, int stage, int grid, cudaStream_t st) {
-  constexpr size_t smem = stage_smem<O, M, kEvolve>();
+  constexpr size_t smem = Layout<O, M, kEvolve>::kBytes;
   static bool configured = false;
   if (!configured) {
     cudaError_t e = cudaFuncSetAttribute(stage_group_kernel<O, M>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
@@ -188,7 +188,7 @@ cudaError_t go_group(const GroupBox* table, const GroupBg& gb, int stage, int gr
 
 template <int O, int M>
 int ctas_per_sm() {
-  constexpr size_t smem = stage_smem<O, M, kEvolve>();
+  constexpr size_t smem = Layout<O, M, kEvolve>::kBytes;
   if (cudaFuncSetAttribute(stage_group_kernel<O, M>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) !=
       cudaSuccess)
     return 1;

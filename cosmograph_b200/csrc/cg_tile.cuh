@@ -9,16 +9,15 @@
 //
 // Bricks and row pitches are chosen so that a warp's tap is free of bank
 // conflicts:
-//   FP64, 4 x 2 x 16: a warp reads two contiguous 16-double rows (two
+//   FP64, 16 points along z: a warp reads two contiguous 16-double rows (two
 //         wavefronts, the minimum for 256 bytes);
-//   FP32, 4 x 4 x 8 with a row pitch of 24 floats: a warp reads four 8-float
-//         row segments whose banks are s, s+24, s+16, s+8 (mod 32), one
-//         wavefront.
+//   FP32, 8 points along z with a row pitch of 24 floats: a warp reads four
+//         8-float row segments whose banks are s, s+24, s+16, s+8 (mod 32),
+//         one wavefront.
 //
-// The copy is software-pipelined by the caller: the next field's elements are
-// fetched into registers while the current tile is being read (Loader), or,
-// with a second tile buffer, copied by cp.async straight into it
-// (AsyncLoader).
+// The copies run asynchronously (cp.async, AsyncLoader, or TMA boxes): the
+// next field's into a second tile buffer where there is one, else while the
+// SM's other CTAs compute.
 #pragma once
 
 namespace cg {
@@ -28,7 +27,7 @@ template <int BX_, int BY_, int BZ_>
 struct Brick {
   static constexpr int BX = BX_, BY = BY_, BZ = BZ_, THREADS = BX * BY * BZ, WARPS = THREADS / 32;
 };
-using Brick64 = Brick<4, 2, 16>;
+using Brick64 = Brick<4, 6, 16>;
 using Brick32 = Brick<4, 4, 8>;
 
 // PITCH: row pitch in elements (0: the copied row length).  ZOFF: tile
@@ -61,7 +60,7 @@ __device__ __forceinline__ int pmod(int v, int n) {
 
 // Global offset of the first element of each tile row, row r = x*TY + y of
 // the brick at (x0, y0): ((x0 - R + x) mod nx, (y0 - R + y) mod ny) * nz.
-// Written by threads r; the caller synchronises the CTA before any Loader
+// Written by threads r; the caller synchronises the CTA before any loader
 // reads them.
 template <class G, class B>
 __device__ __forceinline__ void row_offsets(int x0, int y0, int nx, int ny, int nz, int tid, int* rowoff) {
@@ -102,32 +101,58 @@ struct Loader {
 };
 
 // Asynchronous copy of one field's tile (cp.async, global to shared memory,
-// no register staging), with the lane/row mapping of Loader.  issue() starts
-// this thread's copies and commits them as one group; the caller waits for
-// its groups (cp_async_wait) and synchronises the CTA before reading.
+// no register staging).  Lane l of warp w copies column z = l mod TZU of row
+// (w + WARPS*q)*RPP + l / TZU at step q.  issue() starts this thread's copies
+// and commits them as one group; the caller waits for its groups
+// (cp_async_wait) and synchronises the CTA before reading.
+template <int BYTES>
 __device__ __forceinline__ void cp_async(void* dst, const void* src) {
   const unsigned d = static_cast<unsigned>(__cvta_generic_to_shared(dst));
-  asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(d), "l"(src) : "memory");
+  if constexpr (BYTES == 16)
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(d), "l"(src) : "memory");
+  else
+    asm volatile("cp.async.ca.shared.global [%0], [%1], %2;" ::"r"(d), "l"(src), "n"(BYTES) : "memory");
 }
 __device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
 template <int N>
 __device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory"); }
 
-template <class G, class B>
+// Whole 16-byte groups where every row starts on 16 bytes (nz a multiple of
+// V = 16 / sizeof(T)): the tile's rows then hold whole groups from the aligned
+// column 0 on, and a group never straddles the periodic wrap; a quarter
+// (FP32) or half (FP64) of the instructions.
+template <class G, class B, class T>
 struct AsyncLoader {
+  static constexpr int V = 16 / (int)sizeof(T);
+  static constexpr int C0 = G::CO / V * V;                      // first copied column of the wide form
+  static constexpr int GROUPS = (G::CO + G::TZU - C0 + V - 1) / V;  // groups per row
+  static constexpr int RPPW = 32 / GROUPS;
+  static constexpr int NPWW = (G::ROWS + B::WARPS * RPPW - 1) / (B::WARPS * RPPW);
+  static_assert(C0 + GROUPS * V <= G::TZ && G::TZ % V == 0 && G::ZO % V == 0, "whole groups stay inside a row");
   int row0, col, zoff;  // zoff < 0: lane without a column
+  bool wide;
   __device__ __forceinline__ void init(int tid, int z0, int nz) {
     const int warp = tid >> 5, lane = tid & 31;
-    const int sub = lane / G::TZU;
-    col = lane - sub * G::TZU;
-    row0 = warp * G::RPP + sub;
-    zoff = sub < G::RPP ? pmod(z0 - G::R + col, nz) : -1;
+    wide = nz % V == 0;
+    const int per = wide ? GROUPS : G::TZU, rpp = wide ? RPPW : G::RPP;
+    const int sub = lane / per;
+    col = wide ? C0 + (lane - sub * per) * V : G::CO + lane - sub * per;
+    row0 = warp * rpp + sub;
+    zoff = sub < rpp ? pmod(z0 - G::ZO + col, nz) : -1;
   }
-  __device__ __forceinline__ void issue(double* tl, const double* __restrict__ f, const int* rowoff) const {
+  __device__ __forceinline__ void issue(T* tl, const T* __restrict__ f, const int* rowoff) const {
+    if (wide) {
 #pragma unroll
-    for (int q = 0; q < G::NPW; ++q) {
-      const int r = row0 + B::WARPS * G::RPP * q;
-      if (zoff >= 0 && r < G::ROWS) cp_async(tl + r * G::TZ + G::CO + col, f + rowoff[r] + zoff);
+      for (int q = 0; q < NPWW; ++q) {
+        const int r = row0 + B::WARPS * RPPW * q;
+        if (zoff >= 0 && r < G::ROWS) cp_async<16>(tl + r * G::TZ + col, f + rowoff[r] + zoff);
+      }
+    } else {
+#pragma unroll
+      for (int q = 0; q < G::NPW; ++q) {
+        const int r = row0 + B::WARPS * G::RPP * q;
+        if (zoff >= 0 && r < G::ROWS) cp_async<(int)sizeof(T)>(tl + r * G::TZ + col, f + rowoff[r] + zoff);
+      }
     }
     cp_async_commit();
   }

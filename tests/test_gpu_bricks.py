@@ -1,0 +1,43 @@
+"""Boxes at the edges of the kernels' bricks (FP64 4 x 6 x 16, mixed 4 x 8 x 8
+points of x, y, z): one brick, one point more, whole bricks only, bricks away
+from every face (TMA tiles and flux boxes), odd and even row lengths (wide and
+narrow thread copies).  FP64 bit for bit against the restatement with correctly
+rounded e^x; mixed against FP64."""
+import numpy as np
+import pytest
+
+import oracle
+from cosmograph_b200 import ics, state as S
+from cosmograph_b200.evolution import BoxConfig, evolve
+
+pytestmark = pytest.mark.gpu
+
+SHAPES = [(5, 6, 16), (8, 7, 17), (13, 12, 32), (16, 20, 48), (12, 25, 50)]
+MATTERS = [S.DUST, S.SCALAR, S.VACUUM]
+
+
+@pytest.mark.parametrize("order", [2, 4, 6, 8])
+@pytest.mark.parametrize("case", range(len(SHAPES)))
+def test_fp64_brick_edges_bit_exact(case, order):
+    matter = MATTERS[(case + order // 2) % 3]
+    st = ics.perturbed(SHAPES[case], matter, seed=11 + case, amp=1e-2)
+    ref = oracle.evolve(st, 2, order, lapse="Harmonic", cr=True)
+    got = evolve(st, 2, BoxConfig(order=order, lapse="Harmonic"))
+    differ = [n for f, n in enumerate(st.names) if not np.array_equal(got.fields[f], ref.fields[f])]
+    assert not differ, (SHAPES[case], differ)
+
+
+@pytest.mark.parametrize("order", [2, 4, 6, 8])
+@pytest.mark.parametrize("shape", [(5, 8, 8), (8, 9, 10), (12, 16, 16), (13, 25, 28)])
+def test_mixed_brick_edges(shape, order):
+    """FP32 perturbations of amplitude 1e-3, one step of dt = 0.1 dx: second
+    differences carry 2^-24 / dx^2 relative to the perturbation and enter with
+    dt, so the new state is off by at most about 0.1 * 2^-24 / dx * 4 of it
+    (1e-6 at dx = 1/13 and below), ten times which is allowed."""
+    matter = MATTERS[order // 2 % 3]
+    st = ics.perturbed(shape, matter, seed=3, amp=1e-3)
+    full = evolve(st, 1, BoxConfig(order=order, lapse="Harmonic")).fields
+    got = evolve(st, 1, BoxConfig(order=order, lapse="Harmonic", precision="mixed")).fields
+    for f, n in enumerate(st.names):
+        spread = np.abs(full[f] - full[f].mean()).max()
+        assert np.abs(got[f] - full[f]).max() <= 1e-5 * max(spread, 1e-6), n
