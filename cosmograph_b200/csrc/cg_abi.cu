@@ -956,14 +956,14 @@ int cg_create(const cg_box_desc* boxes, int nboxes, cg_ctx** out) {
       const size_t reg32 = sizeof(float) * (size_t)b.dev.nfields * b.dev.pts;
       if (e == cudaSuccess) e = cudaMalloc(&m.X, reg32);
       if (e == cudaSuccess) e = cudaMalloc(&m.Y, reg32);
-      if (e == cudaSuccess) {
-        cg::mixed::make_tile_maps(m);  // TMA tile copies where the layout allows
-        m.tma = m.tma && ctx->opt_tma;
-      }
       if (e == cudaSuccess && d.matter == CG_MATTER_DUST) {
         const size_t fp = sizeof(float) * (size_t)cg::P_N * b.dev.pts;
         e = cudaMalloc(&m.FP0, fp);
         if (e == cudaSuccess) e = cudaMalloc(&m.FP1, fp);
+      }
+      if (e == cudaSuccess) {
+        cg::mixed::make_tile_maps(m);  // TMA tile copies where the layout allows
+        m.tma = m.tma && ctx->opt_tma;
       }
       for (double* p : {b.dev.P, b.dev.F})
         if (e == cudaSuccess) e = cudaMemset(p, 0, reg);
@@ -1312,6 +1312,30 @@ namespace {
 template <class B>
 int bricks_along(int n, int b) { return (n + b - 1) / b; }
 
+// The GroupBox entries t of a group's members and, after them, the members'
+// flux-primitive maps, into the group's device table.  dev(q): box q's device
+// storage.
+template <class Entry, class Dev>
+int upload_table(cg_ctx* ctx, Group& g, const std::vector<Entry>& t, Dev dev) {
+  static_assert(sizeof(Entry) % alignof(cg::GroupFluxMaps) == 0, "the flux maps after the entries stay aligned");
+  const size_t m = t.size(), tb = sizeof(Entry) * m;
+  std::vector<cg::GroupFluxMaps> fm(m);
+  for (size_t q = 0; q < m; ++q) {
+    const auto& b = dev(g.members[q]);
+    for (int a = 0; a < 3; ++a) {
+      fm[q].fp0[a] = b.fmap0[a];
+      fm[q].fp1[a] = b.fmap1[a];
+    }
+    fm[q].valid = b.fmaps && b.tma;
+  }
+  if (!g.table) CG_CUDA(ctx, cudaMalloc(&g.table, tb + sizeof(cg::GroupFluxMaps) * m));
+  CG_CUDA(ctx, cudaMemcpyAsync(g.table, t.data(), tb, cudaMemcpyHostToDevice, ctx->stream));
+  CG_CUDA(ctx, cudaMemcpyAsync(static_cast<char*>(g.table) + tb, fm.data(), sizeof(cg::GroupFluxMaps) * m,
+                               cudaMemcpyHostToDevice, ctx->stream));
+  CG_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
+  return CG_OK;
+}
+
 // Device table of a group in its launch order (lpt: largest box first).
 int write_table(cg_ctx* ctx, Group& g) {
   std::vector<int> order = g.members;
@@ -1320,7 +1344,7 @@ int write_table(cg_ctx* ctx, Group& g) {
   });
   g.members = order;
   const size_t m = order.size();
-  int first = 0;
+  int first = 0, rc = CG_OK;
   if (g.mixed) {
     using Br = cg::tile::Brick32;
     std::vector<cg::mixed::GroupBox> t(m);
@@ -1341,9 +1365,7 @@ int write_table(cg_ctx* ctx, Group& g) {
       e.first = first;
       first += e.nbx * e.nby * e.nbz;
     }
-    if (!g.table) CG_CUDA(ctx, cudaMalloc(&g.table, sizeof(cg::mixed::GroupBox) * m));
-    CG_CUDA(ctx, cudaMemcpyAsync(g.table, t.data(), sizeof(cg::mixed::GroupBox) * m, cudaMemcpyHostToDevice, ctx->stream));
-    CG_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
+    rc = upload_table(ctx, g, t, [&](int q) -> const cg::MixedBox& { return ctx->boxes[q].mdev; });
   } else {
     using Br = cg::tile::Brick64;
     std::vector<cg::GroupBox> t(m);
@@ -1362,23 +1384,9 @@ int write_table(cg_ctx* ctx, Group& g) {
       e.first = first;
       first += e.nbx * e.nby * e.nbz;
     }
-    // the members' flux-primitive maps follow the GroupBox entries
-    std::vector<cg::GroupFluxMaps> fm(m);
-    for (size_t q = 0; q < m; ++q) {
-      const Box& b = ctx->boxes[order[q]];
-      for (int a = 0; a < 3; ++a) {
-        fm[q].fp0[a] = b.dev.fmap0[a];
-        fm[q].fp1[a] = b.dev.fmap1[a];
-      }
-      fm[q].valid = b.dev.fmaps && b.dev.tma;
-    }
-    const size_t tb = sizeof(cg::GroupBox) * m;
-    if (!g.table) CG_CUDA(ctx, cudaMalloc(&g.table, tb + sizeof(cg::GroupFluxMaps) * m));
-    CG_CUDA(ctx, cudaMemcpyAsync(g.table, t.data(), tb, cudaMemcpyHostToDevice, ctx->stream));
-    CG_CUDA(ctx, cudaMemcpyAsync(static_cast<char*>(g.table) + tb, fm.data(), sizeof(cg::GroupFluxMaps) * m,
-                                 cudaMemcpyHostToDevice, ctx->stream));
-    CG_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
+    rc = upload_table(ctx, g, t, [&](int q) -> const cg::BoxDev& { return ctx->boxes[q].dev; });
   }
+  if (rc) return rc;
   g.total = first;
   return CG_OK;
 }

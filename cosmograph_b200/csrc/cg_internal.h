@@ -44,6 +44,8 @@ struct MixedBox {
   int tma;                 // interior tiles are copied by TMA (maps != 0 and the option on)
   int nx, ny, nz, pts, nfields, order, matter, lapse, normalize;
   int xg;  // ghost planes on each x face (0: periodic box)
+  CUtensorMap fmap0[3], fmap1[3];  // TMA maps of the flux primitives FP0 / FP1 (x, y, z boxes)
+  int fmaps;                       // those maps are encoded
   double dx, dt;
   double ko;     // Kreiss-Oliger coefficient (0: none)
   double* kavg;  // device K_avg - Kbar of the substep input (lapses with K_avg), else null
@@ -61,7 +63,7 @@ struct GroupBox;
 struct GroupBg;
 cudaError_t launch_stage(const MixedBox& b, const Bg& bg, int stage, cudaStream_t st);
 cudaError_t launch_init(const MixedBox& b, const Bg& bg, cudaStream_t st);
-// encode b.mapX / b.mapY and set b.maps = b.tma = 1 when the box allows TMA tile copies
+// encode b.mapX / b.mapY (and b.fmap0 / b.fmap1) and set b.maps = b.tma = 1 when the box allows TMA tile copies
 void make_tile_maps(MixedBox& b);
 // one launch for substep `stage` of every box of a mixed group (as launch_group)
 cudaError_t launch_group(const GroupBox* table, const GroupBg& gb, int order, int matter, int stage, int grid,

@@ -23,6 +23,8 @@
 // Kreiss-Oliger dissipation (orders 2 and 8), a_adj_amp = k_damping_amp = 0.
 #pragma once
 
+#include <type_traits>
+
 #include "cg_group.h"
 #include "cosmograph_b200.h"
 #include "cg_tile.cuh"
@@ -103,18 +105,57 @@ struct GroupBg {
   Bg bg[kMaxGroupBoxes];
 };
 
-// per-thread FP32 slots (same meaning as the FP64 kernel's)
+// per-thread FP32 slots (same meaning as the FP64 kernel's); the matter slots
+// come first, at negative slot numbers
 enum : int {
-  S_DG = 0, S_T1 = 18, S_DPHI = 24, S_DDPHI = 27, S_DA = 33, S_DDA = 36, S_DK = 42,
-  S_DGAM = 45, S_SRC = 54, S_G = 65, S_MAT = 83, S_NSLOT = 87
+  S_DG = 0, S_T1 = 18, S_DPHI = 24, S_DDPHI = 27, S_DA = 33, S_DDA = 36, S_DK = 42, S_END = 45,
+  S_DGAM = S_DPHI,  // d_J Gamma^K until they enter S_T1, before phi and alpha are differentiated
+  S_WIDE = S_T1,    // last substep: the new g and A in FP64, two slots each, after the right-hand sides
 };
-// slots per thread: dust 4 flux divergences, scalar 15 first derivatives
-template <int MATTER>
-struct NSlot {
-  static constexpr int value = S_MAT + (MATTER == kDust ? 4 : (MATTER == kScalar ? 15 : 0));
+// boxes of the dust flux primitives: the brick extended by r along one axis
+// only (z: a tile row, whose pitch keeps a warp's taps on different banks)
+template <int O>
+struct FluxBox {
+  static constexpr int R = O / 2;
+  static constexpr int XB = (kBX + 2 * R) * kBY * kBZ, YB = kBX * (kBY + 2 * R) * kBZ;
+  static constexpr int ZP = TileG<O>::TZ, ZB = kBX * kBY * ZP;
+  static constexpr int SIZE = 5 * (XB + YB + ZB);
 };
-// phase 1 writes no slot in [S_SRC, S_MAT): the field tile lives there
-constexpr int kTileSlot = S_SRC, kTileSlots = S_MAT - S_SRC;
+struct FluxMaps {
+  CUtensorMap m[3];  // x, y and z boxes of the substep input's 7 flux-primitive arrays
+};
+// Shared memory of a CTA, in floats: phase 1 the slots that survive it, then
+// the field tiles (two where CTAS CTAs per SM still fit); the flux boxes lie
+// over the still empty slots.  Phase 2: the sources take the tiles' place.
+template <int O, int MATTER>
+struct Layout {
+  static constexpr int MATN = MATTER == kDust ? 4 : (MATTER == kScalar ? 15 : 0);
+  static constexpr int MAT = -MATN;
+  static constexpr int LIVE = S_END, SRC = LIVE;
+  static constexpr bool FLUX = MATTER == kDust;
+  static constexpr int kSlotEnd = (MATN + LIVE) * kThreads;
+  static constexpr int kFlux = MATN * kThreads;
+  static constexpr int kFluxEnd = FLUX ? kFlux + FluxBox<O>::SIZE : 0;
+  static constexpr int kTile = kSlotEnd > kFluxEnd ? kSlotEnd : kFluxEnd;
+  static constexpr int kTileSize = TileG<O>::SIZE;
+  static constexpr int kRows = (TileG<O>::ROWS + 31) / 32 * 32;  // row offsets of thread copies
+  static constexpr int total(int tiles) {
+    const int a = kTile + tiles * kTileSize + kRows, b = (MATN + LIVE + Q_N) * kThreads;
+    return a > b ? a : b;
+  }
+  // 228 KB per SM, 1 KB reserved per CTA, up to 1 KB of static shared memory
+  static constexpr bool fits(int ctas, int tiles) {
+    return ctas * (total(tiles) * (int)sizeof(float) + 2048) <= 228 * 1024;
+  }
+  static constexpr int CTAS = 2;
+  static constexpr bool TWO = fits(CTAS, 2);
+  static constexpr int kRowOff = kTile + (TWO ? 2 : 1) * kTileSize;
+  static constexpr size_t kBytes = sizeof(float) * (size_t)total(TWO ? 2 : 1);
+  static_assert(fits(CTAS, 1), "two CTAs fit on an SM");
+  static_assert(kFlux % 32 == 0 && kTile % 32 == 0 && kTileSize % 32 == 0 && FluxBox<O>::XB % 32 == 0 &&
+                    FluxBox<O>::YB % 32 == 0 && FluxBox<O>::ZB % 32 == 0,
+                "TMA destinations are 128-byte aligned");
+};
 
 __device__ __forceinline__ int wrapf(int v, int n) {
   v = v < 0 ? v + n : v;
@@ -135,14 +176,6 @@ struct Taps {
     return at((a == 0 ? n : 0) + (b == 0 ? m : 0), (a == 1 ? n : 0) + (b == 1 ? m : 0),
               (a == 2 ? n : 0) + (b == 2 ? m : 0));
   }
-};
-
-// taps of one field read from global memory through index taps T
-template <class T>
-struct GTaps {
-  const float* f;
-  T t;
-  __device__ __forceinline__ float ax(int a, int n) const { return __ldg(f + t.ax(a, n)); }
 };
 
 // FP32 centred stencils (utils/math.h:74-1085 coefficients)
@@ -176,19 +209,11 @@ __device__ __forceinline__ float dm(const T& t, int a, int b, float idx2) {
   else s = 0.4f * P(1) - 0.05f * P(2) + (2.0f / 315.0f) * P(3) - (1.0f / 2240.0f) * P(4);
   return s * idx2;
 }
-template <int O, class T>
-__device__ __forceinline__ float d1p(const float* __restrict__ fa, const float* __restrict__ fb, const T& t, int a,
-                                     float idx) {
-  auto V = [&](int n) {
-    const int q = t.ax(a, n);
-    return __ldg(fa + q) * __ldg(fb + q);
-  };
-  float s;
-  if (O == 2) s = 0.5f * (V(1) - V(-1));
-  else if (O == 4) s = (2.0f / 3.0f) * (V(1) - V(-1)) - (1.0f / 12.0f) * (V(2) - V(-2));
-  else if (O == 6) s = 0.75f * (V(1) - V(-1)) - 0.15f * (V(2) - V(-2)) + (1.0f / 60.0f) * (V(3) - V(-3));
-  else s = 0.8f * (V(1) - V(-1)) - 0.2f * (V(2) - V(-2)) + (4.0f / 105.0f) * (V(3) - V(-3)) - (1.0f / 280.0f) * (V(4) - V(-4));
-  return s * idx;
+// a0 b0 + a1 b1 + a2 b2 with its contractions written out: left to the
+// compiler, a product that another sum shares may stay uncontracted in one
+// kernel (a launch group's) and not in another (a box's own)
+__device__ __forceinline__ float dot3f(float a0, float b0, float a1, float b1, float a2, float b2) {
+  return fmaf(a2, b2, fmaf(a1, b1, a0 * b0));
 }
 
 __device__ __forceinline__ void inv_metricf(const float g[6], float gi[6]) {
@@ -217,114 +242,239 @@ __device__ __forceinline__ DustF dust_primf(const float gi[6], float em4, float 
   return d;
 }
 
-// Phase 1 (as in the FP64 kernel): the metric components, phi and alpha with
-// first and second derivatives, one field tile at a time, the next field
-// fetched into registers meanwhile.  The fields with first derivatives only
-// (K, Gamma^i, the scalar field) read their taps from global memory after
-// the tiles (mixed_body).
-__device__ __forceinline__ int phase1_field(int it) {
-  return it < 6 ? F_G11 + it
-                : (it == 6 ? F_PHI : (it == 7 ? F_ALPHA : (it == 8 ? F_K : (it < 12 ? F_GAM1 + it - 9 : F_SPHI + it - 12))));
-}
+// Fields copied into tiles in phase 1, in the FP64 kernel's order: the metric
+// components with first and second derivatives, Gamma^i with first, phi and
+// alpha with first and second, K with first, (scalar) phi, Pi, psi_i with first.
+template <int MATTER>
+struct Phase1 {
+  static constexpr int GAM = 6, PHI = 9, K = 11, SC = 12, N = SC + (MATTER == kScalar ? 5 : 0);
+  __device__ __forceinline__ static int field(int it) {
+    return it < GAM ? F_G11 + it
+                    : (it < PHI ? F_GAM1 + it - GAM
+                                : (it == PHI ? F_PHI : (it < K ? F_ALPHA : (it == K ? F_K : F_SPHI + it - SC))));
+  }
+};
 
-// first and second derivatives of phase-1 field `it` from its tile
-template <int O, class T>
-__device__ __forceinline__ void field_derivatives(int it, const T& t, float idx, float idx2, const float gi[6],
-                                                  float* sl) {
-  {
-    if (it < 8) {
-      const float g1 = d1<O>(t, 0, idx), g2 = d1<O>(t, 1, idx), g3 = d1<O>(t, 2, idx);
-      const float h11 = d2<O>(t, 0, idx2), h22 = d2<O>(t, 1, idx2), h33 = d2<O>(t, 2, idx2);
-      const float h12 = dm<O>(t, 0, 1, idx2), h13 = dm<O>(t, 0, 2, idx2), h23 = dm<O>(t, 1, 2, idx2);
-      if (it < 6) {
-        sl[(S_DG + 0 * 6 + it) * kThreads] = g1;
-        sl[(S_DG + 1 * 6 + it) * kThreads] = g2;
-        sl[(S_DG + 2 * 6 + it) * kThreads] = g3;
-        sl[(S_T1 + it) * kThreads] =
-            gi[0] * h11 + gi[3] * h22 + gi[5] * h33 + 2.0f * (gi[1] * h12 + gi[2] * h13 + gi[4] * h23);
-      } else {
-        const int b1 = it == 6 ? S_DPHI : S_DA, b2 = it == 6 ? S_DDPHI : S_DDA;
-        sl[(b1 + 0) * kThreads] = g1;
-        sl[(b1 + 1) * kThreads] = g2;
-        sl[(b1 + 2) * kThreads] = g3;
-        sl[(b2 + 0) * kThreads] = h11;
-        sl[(b2 + 1) * kThreads] = h12;
-        sl[(b2 + 2) * kThreads] = h13;
-        sl[(b2 + 3) * kThreads] = h22;
-        sl[(b2 + 4) * kThreads] = h23;
-        sl[(b2 + 5) * kThreads] = h33;
-      }
+// the derivatives of phase-1 field `it` from its tile, into the slots
+template <int O, int MATTER, class T>
+__device__ __forceinline__ void field_derivatives(int it, const T& t, float idx, float idx2, const float g[6],
+                                                  const float gi[6], float* sl) {
+  using PF = Phase1<MATTER>;
+  auto S = [&](int s) -> float& { return sl[s * kThreads]; };
+  const float d[3] = {d1<O>(t, 0, idx), d1<O>(t, 1, idx), d1<O>(t, 2, idx)};
+  if (it < PF::GAM || (it >= PF::PHI && it < PF::K)) {
+    const float h11 = d2<O>(t, 0, idx2), h22 = d2<O>(t, 1, idx2), h33 = d2<O>(t, 2, idx2);
+    const float h12 = dm<O>(t, 0, 1, idx2), h13 = dm<O>(t, 0, 2, idx2), h23 = dm<O>(t, 1, 2, idx2);
+    if (it < PF::GAM) {
+#pragma unroll
+      for (int x = 0; x < 3; ++x) S(S_DG + x * 6 + it) = d[x];
+      S(S_T1 + it) = gi[0] * h11 + gi[3] * h22 + gi[5] * h33 + 2.0f * (gi[1] * h12 + gi[2] * h13 + gi[4] * h23);
+    } else {
+      const int b1 = it == PF::PHI ? S_DPHI : S_DA, b2 = it == PF::PHI ? S_DDPHI : S_DDA;
+#pragma unroll
+      for (int x = 0; x < 3; ++x) S(b1 + x) = d[x];
+      S(b2 + 0) = h11;
+      S(b2 + 1) = h12;
+      S(b2 + 2) = h13;
+      S(b2 + 3) = h22;
+      S(b2 + 4) = h23;
+      S(b2 + 5) = h33;
     }
+    return;
+  }
+  const int b = it < PF::PHI ? S_DGAM + 3 * (it - PF::GAM) : (it == PF::K ? S_DK : Layout<O, MATTER>::MAT + 3 * (it - PF::SC));
+#pragma unroll
+  for (int x = 0; x < 3; ++x) S(b + x) = d[x];
+  if (it == PF::PHI - 1) {
+    // all of d_J Gamma^K: Ricci term 2 (bssn_macros.h:251-252) joins term 1;
+    // phi and alpha then take the slots
+    float gm[6], dG[9], B[3][3];
+#pragma unroll
+    for (int m = 0; m < 6; ++m) gm[m] = (m == 0 || m == 3 || m == 5) ? g[m] + 1.0f : g[m];
+#pragma unroll
+    for (int m = 0; m < 9; ++m) dG[m] = S(S_DGAM + m);
+#pragma unroll
+    for (int I = 0; I < 3; ++I)
+#pragma unroll
+      for (int J = 0; J < 3; ++J) B[I][J] = gm[sym(0, I)] * dG[J] + gm[sym(1, I)] * dG[3 + J] + gm[sym(2, I)] * dG[6 + J];
+#pragma unroll
+    for (int I = 0; I < 3; ++I)
+#pragma unroll
+      for (int J = I; J < 3; ++J) S(S_T1 + sym(I, J)) = 0.5f * (B[I][J] + B[J][I] - S(S_T1 + sym(I, J)));
   }
 }
 
-// The tile copies: by TMA (tmap != null, a brick whose halo lies inside the
-// box) or by the threads' own loads with periodic wrap.  Returns false (the
-// same value in every thread) when a TMA copy did not complete within
-// tma_wait cycles; the status word then carries kStatusTileTimeout.  A late
-// copy is still waited for (tma::wait_drain), so that none is in flight when
-// the tile is reused or the CTA leaves; after a copy that never lands the CTA
-// issues no more.
+// dust flux divergences d_i(alpha D v^i), d_i(alpha S_m v^i) (dust.cc:203-224)
+// into the matter slots, one axis at a time in a rolled loop; axis(a): the taps
+// of axis a, (m, n) -> the value at offset n of alpha*D, alpha*S_1..3 (m < 4)
+// or v^a (m = 4), the latter read once for the four sums
+template <int O, class T>
+struct FluxTaps {
+  const T& t;
+  const float* v;
+  int m;
+  __device__ __forceinline__ float ax(int, int n) const { return t(m, n) * v[n < 0 ? n + O / 2 : O / 2 + n - 1]; }
+};
+template <int O, class AxisOf>
+__device__ __forceinline__ void flux_divergences(AxisOf axis, float idx, float* mat) {
+  constexpr int R = O / 2;
+  float div[4] = {0.f, 0.f, 0.f, 0.f};
+#pragma unroll 1
+  for (int a = 0; a < 3; ++a) {
+    const auto t = axis(a);
+    float v[2 * R];
+#pragma unroll
+    for (int n = 0; n < R; ++n) {
+      v[n] = t(4, n - R);
+      v[R + n] = t(4, n + 1);
+    }
+#pragma unroll
+    for (int m = 0; m < 4; ++m) div[m] += d1<O>(FluxTaps<O, decltype(t)>{t, v, m}, 0, idx);
+  }
+#pragma unroll
+  for (int m = 0; m < 4; ++m) mat[m * kThreads] = div[m];
+}
+// taps of one axis in its five staged boxes of len values, stride st
+struct BoxAxis {
+  const float* u;
+  int len, st;
+  __device__ __forceinline__ float operator()(int m, int n) const { return u[m * len + n * st]; }
+};
+// taps of one axis in global memory: u alpha*D at the point, v its v^a, off[]
+// the (periodic) offsets -R..-1, 1..R
+template <int O>
+struct GlobalAxis {
+  const float *u, *v;
+  size_t N;
+  int off[O];
+  __device__ __forceinline__ float operator()(int m, int n) const {
+    return __ldg((m < 4 ? u + m * N : v) + off[n < 0 ? n + O / 2 : O / 2 + n - 1]);
+  }
+};
+
+// Phase 1, as in the FP64 kernel.  The tile copies: by TMA (tmap != null, a
+// brick whose halo lies inside the box) or by the threads' cp.async with
+// periodic wrap.  Returns false (the same value in every thread) when a TMA
+// copy did not complete within tma_wait cycles; the status word then carries
+// kStatusTileTimeout.  A late copy is still waited for (tma::wait_drain), so
+// that none is in flight when a buffer is reused or the CTA leaves; after a
+// copy that never lands the CTA issues no more.  bar[0], bar[1]: mbarriers of
+// the tile buffers, bar[2] of the flux boxes; bit b of phase is the parity
+// bar[b] completes next.
 template <int O, int MATTER>
 __device__ __forceinline__ bool derivatives(const float* __restrict__ a, int N, float idx, float idx2,
-                                            const float gi[6], float* sl, float* tl, const int* rowoff, int tid,
-                                            int x0, int y0, int z0, int nz, int cc, const CUtensorMap* tmap,
-                                            uint64_t* bar, unsigned& phase, unsigned* status, long long tma_wait) {
+                                            const float g[6], const float gi[6], float* smem, float* sl, int tid,
+                                            int x0, int y0, int z0, int tx, int ty, int tz, int nz,
+                                            const CUtensorMap* tmap, const FluxMaps* fm, uint64_t* bar,
+                                            unsigned& phase, unsigned* status, long long tma_wait) {
+  using PF = Phase1<MATTER>;
+  using L = Layout<O, MATTER>;
   using G = TileG<O>;
-  const tile::Taps<G, float> t{tl, cc};
-  constexpr int NIT = 8;  // fields with second derivatives; first-derivative-only fields use global taps
-  const bool by_tma = tmap != nullptr;
+  using FB = FluxBox<O>;
+  constexpr bool TWO = L::TWO;
+  float* tl = smem + L::kTile;
+  float* tl2 = tl + (TWO ? L::kTileSize : 0);
+  const int* rowoff = reinterpret_cast<const int*>(smem + L::kRowOff);
+  const int cc = tile::centre<G>(tx, ty, tz);
+  unsigned pending = 0;
+  auto issue = [&](int it) {
+    const int b = TWO ? (it & 1) : 0;
+    if (tid == 0) {
+      tma::arrive_expect_tx(bar + b, (unsigned)(G::SIZE * sizeof(float)));
+      tma::load_4d(b ? tl2 : tl, tmap, z0 - G::ZO, y0 - G::R, x0 - G::R, PF::field(it), bar + b);
+      if (it + 1 < PF::N) tma::prefetch_4d(tmap, z0 - G::ZO, y0 - G::R, x0 - G::R, PF::field(it + 1));
+    }
+    pending |= 1u << b;
+  };
   bool ok = true, lost = false;
-  tile::Loader<G, Brick, float> ld;
-  if (!by_tma) {
-    ld.init(tid, z0, nz);
-    ld.fetch(a + (size_t)phase1_field(0) * N, rowoff);
+  auto wait = [&](int b) {
+    if (!(pending & (1u << b))) return;
+    const int w = tma::wait_drain(bar + b, (phase >> b) & 1u, tma_wait);
+    ok = ok && w == 0;
+    pending &= ~(1u << b);
+    if (w == 2) lost = true;
+    else phase ^= 1u << b;
+  };
+  const bool by_tma = tmap != nullptr;
+  tile::AsyncLoader<G, Brick, float> ald;
+  if (by_tma) {
+    tma::fence_proxy_async();  // this thread's shared-memory accesses come before the copies' writes
+    __syncthreads();
+    if constexpr (L::FLUX) {
+      if (fm) {
+        float* box = smem + L::kFlux;
+        if (tid == 0) {
+          tma::arrive_expect_tx(bar + 2, (unsigned)(FB::SIZE * sizeof(float)));
+          for (int ax = 0; ax < 3; ++ax) {
+            const int len = ax == 0 ? FB::XB : (ax == 1 ? FB::YB : FB::ZB);
+            for (int q = 0; q < 5; ++q, box += len)  // alpha*D, alpha*S_1..3, then v^a
+              tma::load_4d(box, &fm->m[ax], z0 - (ax == 2 ? G::ZO : 0), y0 - (ax == 1 ? FB::R : 0),
+                           x0 - (ax == 0 ? FB::R : 0), q < 4 ? P_AD + q : P_V1 + ax, bar + 2);
+          }
+        }
+        pending |= 4u;
+      }
+    }
+    issue(0);
+    if constexpr (L::FLUX) {
+      if (fm) {
+        const float* box = smem + L::kFlux;
+        wait(2);
+        flux_divergences<O>(
+            [&](int ax) {
+              const int c = ax == 0   ? ((tx + FB::R) * kBY + ty) * kBZ + tz
+                            : ax == 1 ? 5 * FB::XB + (tx * (kBY + 2 * FB::R) + ty + FB::R) * kBZ + tz
+                                      : 5 * (FB::XB + FB::YB) + (tx * kBY + ty) * FB::ZP + tz + G::ZO;
+              return BoxAxis{box + c, ax == 0 ? FB::XB : (ax == 1 ? FB::YB : FB::ZB),
+                             ax == 0 ? kBY * kBZ : (ax == 1 ? kBZ : 1)};
+            },
+            idx, sl + L::MAT * kThreads);
+      }
+    }
+  } else {
+    ald.init(tid, z0, nz);
+    ald.issue(tl, a + (size_t)PF::field(0) * N, rowoff);
   }
   // one loop (and one copy of the derivative code) for both kinds of copy
 #pragma unroll 1
-  for (int it = 0; it < NIT; ++it) {
+  for (int it = 0; it < PF::N; ++it) {
+    const int b = TWO ? (it & 1) : 0;
+    // the buffer that the next copy writes has been read (first pass: the flux boxes, which the slots overwrite)
     if (by_tma) {
-      tma::fence_proxy_async();        // this thread's shared-memory accesses come before the copy's writes
-      lost = __syncthreads_or(lost);   // the previous tile has been read
+      tma::fence_proxy_async();
+      lost = __syncthreads_or(lost);
       if (!lost) {
-        if (tid == 0) {
-          tma::arrive_expect_tx(bar, (unsigned)(G::SIZE * sizeof(float)));
-          tma::load_4d(tl, tmap, z0 - G::ZO, y0 - G::R, x0 - G::R, phase1_field(it), bar);
-          // the next field's tile into L2 while this one is used
-          if (it + 1 < NIT) tma::prefetch_4d(tmap, z0 - G::ZO, y0 - G::R, x0 - G::R, phase1_field(it + 1));
+        if (TWO) {
+          if (it + 1 < PF::N) issue(it + 1);
+        } else if (it > 0) {
+          issue(it);
         }
-        const int w = tma::wait_drain(bar, phase, tma_wait);
-        ok = ok && w == 0;
-        if (w == 2) lost = true;
-        else phase ^= 1u;
       }
+      wait(b);
     } else {
       __syncthreads();
-      ld.store(tl);
+      if (TWO) {
+        if (it + 1 < PF::N) {
+          ald.issue((it + 1) & 1 ? tl2 : tl, a + (size_t)PF::field(it + 1) * N, rowoff);
+          tile::cp_async_wait<1>();
+        } else {
+          tile::cp_async_wait<0>();
+        }
+      } else {
+        if (it > 0) ald.issue(tl, a + (size_t)PF::field(it) * N, rowoff);
+        tile::cp_async_wait<0>();
+      }
       __syncthreads();
-      if (it + 1 < NIT) ld.fetch(a + (size_t)phase1_field(it + 1) * N, rowoff);
     }
-    field_derivatives<O>(it, t, idx, idx2, gi, sl);
+    field_derivatives<O, MATTER>(it, tile::Taps<G, float>{b ? tl2 : tl, cc}, idx, idx2, g, gi, sl);
   }
   if (by_tma) {
+    wait(0);  // after a lost copy: the other buffer's copy in flight
+    wait(1);
     ok = __syncthreads_and(ok && !lost);
     if (!ok && tid == 0) atomicOr(status, kStatusTileTimeout);
   }
   return ok;
-}
-
-// dust flux divergences from the stored FP32 flux primitives (global taps)
-template <int O, class T>
-__device__ __forceinline__ void flux_divergences(const T& t, const float* __restrict__ fp, int N, float idx,
-                                                 float* sl) {
-  const float* v1 = fp + (size_t)P_V1 * N;
-  const float* v2 = fp + (size_t)P_V2 * N;
-  const float* v3 = fp + (size_t)P_V3 * N;
-#pragma unroll 1
-  for (int m = 0; m < 4; ++m) {
-    const float* u = fp + (size_t)(P_AD + m) * N;
-    sl[(S_MAT + m) * kThreads] = d1p<O>(u, v1, t, 0, idx) + d1p<O>(u, v2, t, 1, idx) + d1p<O>(u, v3, t, 2, idx);
-  }
 }
 
 // dalpha/dt(abar + delta) - dalpha/dt(abar) for the lapse gauges of
@@ -372,13 +522,16 @@ template <int O, int MATTER, bool KO = false>
 __device__ __forceinline__ void mixed_body(int nx, int ny, int nz, int lapse, int normalize, float idx, double dt,
                                            const Bg& bg, const Ptrs& P, int stage, int cx, int cy, int cz,
                                            const CUtensorMap* tmap, uint64_t* bar, unsigned& phase,
-                                           bool& tma_ok) {
+                                           bool& tma_ok, const FluxMaps* fmaps) {
+  using L = Layout<O, MATTER>;
+  constexpr int MAT = L::MAT, SRC = L::SRC;
   constexpr int NFLD = MATTER == kDust ? 22 : (MATTER == kScalar ? 23 : 18);
   constexpr int R = O / 2;
   constexpr float kPif = 3.14159265358979f;
   extern __shared__ __align__(128) float smf[];  // 128-byte aligned: TMA destinations
+  __shared__ double bg_rhs[NFLD], bg_out[NFLD];  // the uniform background of each field, for the rolled epilogue
   const int tid = threadIdx.x + kBZ * (threadIdx.y + kBY * threadIdx.z);
-  float* sl = smf + tid;
+  float* sl = smf + L::MATN * kThreads + tid;  // this thread's slot column
   auto S = [&](int s) -> float& { return sl[s * kThreads]; };
   const int k0 = cz * kBZ + threadIdx.x;
   const int j0 = cy * kBY + threadIdx.y;
@@ -390,13 +543,30 @@ __device__ __forceinline__ void mixed_body(int nx, int ny, int nz, int lapse, in
   const int N = nx * ny * nz;
   const int c = (i * ny + j) * nz + k;
   const float* __restrict__ a = P.in;
-  auto D_ = [&](int f) { return a[(size_t)f * N + c]; };  // delta at the centre
+  // element c of field f of a block: the field's address is the same for the
+  // whole CTA, the thread's part a 32-bit byte offset (fields of at most 2^28
+  // points: a box's registers of more would not fit the GPU)
+  const unsigned c4 = (unsigned)c * 4u, c8 = (unsigned)c * 8u;
+  auto fat = [&](auto* block, int f) { return reinterpret_cast<decltype(block)>((uintptr_t)(block + (size_t)f * N) + (sizeof(*block) == 4 ? c4 : c8)); };
+  auto D_ = [&](int f) { return *fat(a, f); };  // delta at the centre
+  const int x0 = cx * kBX, y0 = cy * kBY, z0 = cz * kBZ;
   // warm L2 with the epilogue's FP64 register reads; those reads and the
-  // epilogue writes are single-use streams (ld/st .cs), as in the FP64 kernel
+  // epilogue writes are single-use streams (ld/st .cs); one prefetch per
+  // 32-byte sector of the brick's rows, as in the FP64 kernel
+  {
+    constexpr int SEC = kBZ / 4 + 1, PER = kBX * kBY * SEC, GRP = kThreads / PER;  // a field's sectors, fields at a time
+    if (tid < GRP * PER) {
+      const int b = tid % PER, row = b / SEC;
+      const int x = min(x0 + row / kBY, nx - 1), y = min(y0 + row % kBY, ny - 1);
+      const int z = min(z0 + 4 * (b % SEC), min(z0 + kBZ, nz) - 1);
+      const size_t at = (size_t)(tid / PER) * N + ((x * ny + y) * nz + z);
 #pragma unroll 1
-  for (int f = 0; f < NFLD; ++f) {
-    asm volatile("prefetch.global.L2 [%0];" :: "l"(P.p + (size_t)f * N + c));
-    if (stage > 1) asm volatile("prefetch.global.L2 [%0];" :: "l"(P.f + (size_t)f * N + c));
+      for (int reg = 0; reg < (stage > 1 ? 2 : 1); ++reg) {
+        const double* q = (reg ? P.f : P.p) + at;
+#pragma unroll 4
+        for (int f = tid / PER; f < NFLD; f += GRP, q += (size_t)GRP * N) asm volatile("prefetch.global.L2 [%0];" :: "l"(q));
+      }
+    }
   }
 
   float g[6], gi[6];
@@ -404,47 +574,43 @@ __device__ __forceinline__ void mixed_body(int nx, int ny, int nz, int lapse, in
   for (int q = 0; q < 6; ++q) g[q] = D_(F_G11 + q);
   inv_metricf(g, gi);
 
-  const int x0 = cx * kBX, y0 = cy * kBY, z0 = cz * kBZ;
+  // read after the barriers of phase 1
+  if (tid < NFLD) {
+    const int b = tid == F_K ? 0 : (tid == F_PHI ? 1 : (tid == F_ALPHA ? 2 : (tid == 18 ? 3 : (tid == 19 ? 4 : -1))));
+    bg_rhs[tid] = b < 0 ? 0.0 : bg.rhs[b];
+    bg_out[tid] = b < 0 ? 0.0 : bg.out[b];
+  }
   const float idx2 = idx * idx;
+  bool flux_tiles = false;  // the dust flux divergences came from TMA boxes
   {
-    static_assert(TileG<O>::SIZE * sizeof(float) + TileG<O>::ROWS * sizeof(int) <=
-                      (size_t)kTileSlots * kThreads * sizeof(float),
-                  "tile and row offsets fit the phase-2-only slots");
     using G = TileG<O>;
-    float* tl = smf + kTileSlot * kThreads;
-    int* rowoff = reinterpret_cast<int*>(tl + G::SIZE);
     // TMA when the brick's halo lies inside the box (no wrap)
     const bool by_tma = tmap && tma_ok && x0 >= G::R && x0 + kBX + G::R <= nx && y0 >= G::R && y0 + kBY + G::R <= ny &&
                         z0 >= G::ZO && z0 + kBZ + G::R <= nz;
     if (!by_tma) {
-      tile::row_offsets<G, Brick>(x0, y0, nx, ny, nz, tid, rowoff);
+      tile::row_offsets<G, Brick>(x0, y0, nx, ny, nz, tid, reinterpret_cast<int*>(smf + L::kRowOff));
       __syncthreads();  // every warp reads every row offset
     }
+    flux_tiles = L::FLUX && fmaps && by_tma;
     // after a copy timed out the CTA copies by threads (the barrier's phase is unknown)
-    tma_ok = derivatives<O, MATTER>(a, N, idx, idx2, gi, sl, tl, rowoff, tid, x0, y0, z0, nz,
-                                    tile::centre<G>(threadIdx.z, threadIdx.y, threadIdx.x), by_tma ? tmap : nullptr,
-                                    bar, phase, P.status, bg.tma_wait) && tma_ok;
-    __syncthreads();
+    tma_ok = derivatives<O, MATTER>(a, N, idx, idx2, g, gi, smf, sl, tid, x0, y0, z0, threadIdx.z, threadIdx.y,
+                                    threadIdx.x, nz, by_tma ? tmap : nullptr, flux_tiles ? fmaps : nullptr, bar,
+                                    phase, P.status, bg.tma_wait) && tma_ok;
+    __syncthreads();  // the tiles become slots again
   }
   if (!live) return;
-  {
-    const bool interior =
-        x0 >= R && x0 + kBX + R <= nx && y0 >= R && y0 + kBY + R <= ny && z0 >= R && z0 + kBZ + R <= nz;
-    auto gpass = [&](auto t) {
-      constexpr int NG = MATTER == kScalar ? 9 : 4;  // K, Gamma^i (and phi_s, Pi, psi_i)
-#pragma unroll 1
-      for (int q = 0; q < NG; ++q) {
-        const int fld = q == 0 ? F_K : (q < 4 ? F_GAM1 + q - 1 : F_SPHI + q - 4);
-        const int b = q == 0 ? S_DK : (q < 4 ? S_DGAM + 3 * (q - 1) : S_MAT + 3 * (q - 4));
-        const GTaps<decltype(t)> gt{a + (size_t)fld * N, t};
-        S(b + 0) = d1<O>(gt, 0, idx);
-        S(b + 1) = d1<O>(gt, 1, idx);
-        S(b + 2) = d1<O>(gt, 2, idx);
-      }
-      if (MATTER == kDust) flux_divergences<O>(t, P.fp_in, N, idx, sl);
-    };
-    if (interior) gpass(Taps<false>{i, j, k, nx, ny, nz, ny * nz, nz, c});
-    else gpass(Taps<true>{i, j, k, nx, ny, nz, ny * nz, nz, c});
+  if (MATTER == kDust && !flux_tiles) {
+    // flux taps from global memory
+    flux_divergences<O>(
+        [&](int ax) {
+          const int at = ax == 0 ? i : (ax == 1 ? j : k), n = ax == 0 ? nx : (ax == 1 ? ny : nz);
+          const int st = ax == 0 ? ny * nz : (ax == 1 ? nz : 1);
+          GlobalAxis<O> t{P.fp_in + (size_t)P_AD * N + c, P.fp_in + (size_t)(P_V1 + ax) * N + c, (size_t)N, {}};
+#pragma unroll
+          for (int q = 0; q < O; ++q) t.off[q] = (wrapf(at + (q < R ? q - R : q - R + 1), n) - at) * st;
+          return t;
+        },
+        idx, sl + MAT * kThreads);
   }
 
   // ---- centre values: perturbations and full values -------------------------
@@ -473,12 +639,12 @@ __device__ __forceinline__ void mixed_body(int nx, int ny, int nz, int lapse, in
     } else {
       const float* pv = P.prev;
 #pragma unroll
-      for (int m = 0; m < 6; ++m) gl[m] = __ldcs(&pv[(size_t)(F_G11 + m) * N + c]);
+      for (int m = 0; m < 6; ++m) gl[m] = __ldcs(fat(pv, F_G11 + m));
       inv_metricf(gl, gil);
-      dphil = __ldcs(&pv[(size_t)F_PHI * N + c]);
+      dphil = __ldcs(fat(pv, F_PHI));
       phil = (float)bgv(bg.prev, F_PHI) + dphil;
-      Dl = (float)bgv(bg.prev, F_D) + __ldcs(&pv[(size_t)F_D * N + c]);
-      Sl[0] = __ldcs(&pv[(size_t)F_S1 * N + c]); Sl[1] = __ldcs(&pv[(size_t)F_S2 * N + c]); Sl[2] = __ldcs(&pv[(size_t)F_S3 * N + c]);
+      Dl = (float)bgv(bg.prev, F_D) + __ldcs(fat(pv, F_D));
+      Sl[0] = __ldcs(fat(pv, F_S1)); Sl[1] = __ldcs(fat(pv, F_S2)); Sl[2] = __ldcs(fat(pv, F_S3));
     }
     const float em4l = __expf(-4.0f * phil), e6l = __expf(6.0f * phil), e4l = __expf(4.0f * phil);
     const DustF dl = dust_primf(gil, em4l, e6l, Dl, Sl);
@@ -488,19 +654,19 @@ __device__ __forceinline__ void mixed_body(int nx, int ny, int nz, int lapse, in
     const float inv_detg = 1.0f / e6l;
     Sdust = D * inv_detg * dl.w2 / dl.W;
     rS_full = (float)(bgv(bg.in, F_D) * bg.e6l) + dr + Sdust - 2.0f * (float)bg.lambda;
-    S(S_SRC + Q_R) = dr;
-    S(S_SRC + Q_S) = Sdust;
+    S(SRC + Q_R) = dr;
+    S(SRC + Q_S) = Sdust;
 #pragma unroll
-    for (int m = 0; m < 3; ++m) S(S_SRC + Q_S1 + m) = Sv[m] * inv_detg;
+    for (int m = 0; m < 3; ++m) S(SRC + Q_S1 + m) = Sv[m] * inv_detg;
 #pragma unroll
     for (int I = 0; I < 3; ++I)
 #pragma unroll
       for (int J = I; J < 3; ++J)
-        S(S_SRC + Q_STF11 + sym(I, J)) = Sv[I] * Sv[J] / (dl.W * D) * inv_detg - (1.0f / 3.0f) * (e4l * (gl[sym(I, J)] + (I == J ? 1.0f : 0.0f))) * Sdust;
+        S(SRC + Q_STF11 + sym(I, J)) = Sv[I] * Sv[J] / (dl.W * D) * inv_detg - (1.0f / 3.0f) * (e4l * (gl[sym(I, J)] + (I == J ? 1.0f : 0.0f))) * Sdust;
     // dust RHS: divergence + momentum source with the current W, v (dust.cc:135-146)
     const DustF cur = dust_primf(gi, em4phi, __expf(6.0f * phi), D, Sv);
     const float e4 = __expf(4.0f * phi);
-    rhs_m[0] = S(S_MAT + 0);
+    rhs_m[0] = S(MAT + 0);
 #pragma unroll
     for (int d = 0; d < 3; ++d) {
       const float dp = S(S_DPHI + d);
@@ -512,7 +678,7 @@ __device__ __forceinline__ void mixed_body(int nx, int ny, int nz, int lapse, in
                2.0f * (cur.v[0] * cur.v[1] * (4.0f * gm[1] * dp + DG(1)) + cur.v[0] * cur.v[2] * (4.0f * gm[2] * dp + DG(2)) +
                        cur.v[1] * cur.v[2] * (4.0f * gm[4] * dp + DG(4)))) -
           cur.W * D * S(S_DA + d);
-      rhs_m[1 + d] = S(S_MAT + 1 + d) + src;
+      rhs_m[1 + d] = S(MAT + 1 + d) + src;
     }
   } else if (MATTER == kScalar) {
     // Scalar::addBSSNSource and RKEvolvePt (scalar.cc:85-260) in perturbation
@@ -524,7 +690,7 @@ __device__ __forceinline__ void mixed_body(int nx, int ny, int nz, int lapse, in
     const float dsphi = D_(F_SPHI), dPi = D_(F_SPI);
     const float sphi = sphib + dsphi, Pi = Pib + dPi;
     const float psi[3] = {D_(F_SPSI1), D_(F_SPSI1 + 1), D_(F_SPSI1 + 2)};
-    auto SD = [&](int m, int d) { return S(S_MAT + 3 * m + d); };  // d_d of scalar field m
+    auto SD = [&](int m, int d) { return S(MAT + 3 * m + d); };  // d_d of scalar field m
     const float dd = gi[0] * SD(0, 0) * SD(0, 0) + gi[3] * SD(0, 1) * SD(0, 1) + gi[5] * SD(0, 2) * SD(0, 2) +
                      2.0f * (gi[1] * SD(0, 0) * SD(0, 1) + gi[2] * SD(0, 0) * SD(0, 2) + gi[4] * SD(0, 1) * SD(0, 2));
     const bool quad = bg.potential == kPotQuadratic;
@@ -535,13 +701,13 @@ __device__ __forceinline__ void mixed_body(int nx, int ny, int nz, int lapse, in
     dr = 2.0f * dPi2 - 2.0f * dV;  // delta(rho + S); the dd terms cancel
     Sdust = 0.0f;
     rS_full = 2.0f * Pi * Pi - 2.0f * V;
-    S(S_SRC + Q_R) = 0.5f * dPi2 + 0.5f * em4phi * dd + dV;
+    S(SRC + Q_R) = 0.5f * dPi2 + 0.5f * em4phi * dd + dV;
 #pragma unroll
-    for (int m = 0; m < 3; ++m) S(S_SRC + Q_S1 + m) = Pi * SD(0, m);
+    for (int m = 0; m < 3; ++m) S(SRC + Q_S1 + m) = Pi * SD(0, m);
 #pragma unroll
     for (int I = 0; I < 3; ++I)
 #pragma unroll
-      for (int J = I; J < 3; ++J) S(S_SRC + Q_STF11 + sym(I, J)) = SD(0, I) * SD(0, J) - gm[sym(I, J)] * (1.0f / 3.0f) * dd;
+      for (int J = I; J < 3; ++J) S(SRC + Q_STF11 + sym(I, J)) = SD(0, I) * SD(0, J) - gm[sym(I, J)] * (1.0f / 3.0f) * dd;
     float inner = 0.0f;
 #pragma unroll
     for (int X = 0; X < 3; ++X)
@@ -562,62 +728,83 @@ __device__ __forceinline__ void mixed_body(int nx, int ny, int nz, int lapse, in
     for (int m = 0; m < 3; ++m) rhs_m[2 + m] = -alpha * SD(1, m) - Pi * S(S_DA + m);
   } else {
 #pragma unroll
-    for (int m = 0; m < Q_N; ++m) S(S_SRC + m) = 0.f;
+    for (int m = 0; m < Q_N; ++m) S(SRC + m) = 0.f;
   }
 
-  // ---- Christoffels, D_iD_j phi, (D_iD_j alpha)^TF, Ricci (first order) ---------
+  // Right-hand sides are parked in slots as they are formed (the matter
+  // fields' in the matter slots, the BSSN fields' in the lowered symbols' after
+  // the Ricci tensor), and one rolled loop below updates every register.
+  constexpr int NM = NFLD - F_D;
+  auto cvslot = [](int fld) { return fld < F_D ? S_DG + fld : L::MAT + fld - F_D; };
 #pragma unroll
-  for (int I = 0; I < 3; ++I)
+  for (int m = 0; m < NM; ++m) S(cvslot(F_D + m)) = rhs_m[m];
+
+  // ---- A^ij, Christoffels, D_iD_j phi, (D_iD_j alpha)^TF and Gamma^i -------------
+  float A[6], Ac[6];
+#pragma unroll
+  for (int q = 0; q < 6; ++q) A[q] = D_(F_A11 + q);
+#pragma unroll
+  for (int I = 0; I < 3; ++I) {
+    // g^{IX} A_{XY}, then raised again
+    float m[3];
+#pragma unroll
+    for (int Y = 0; Y < 3; ++Y) m[Y] = dot3f(gi[sym(I, 0)], A[sym(0, Y)], gi[sym(I, 1)], A[sym(1, Y)], gi[sym(I, 2)], A[sym(2, Y)]);
+#pragma unroll
+    for (int J = I; J < 3; ++J) Ac[sym(I, J)] = dot3f(m[0], gi[sym(J, 0)], m[1], gi[sym(J, 1)], m[2], gi[sym(J, 2)]);
+  }
+  const float AijAij = fmaf(2.0f, dot3f(Ac[1], A[1], Ac[2], A[2], Ac[4], A[4]), dot3f(Ac[0], A[0], Ac[3], A[3], Ac[5], A[5]));
+  float dphi[3], da[3];
+#pragma unroll
+  for (int d = 0; d < 3; ++d) { dphi[d] = S(S_DPHI + d); da[d] = S(S_DA + d); }
+  float DDa[6], gld[3], Gd[3], so[3], gldda = 0.f;
+#pragma unroll
+  for (int I = 0; I < 3; ++I) gld[I] = dot3f(gi[sym(I, 0)], dphi[0], gi[sym(I, 1)], dphi[1], gi[sym(I, 2)], dphi[2]);
+#pragma unroll
+  for (int I = 0; I < 3; ++I) gldda = fmaf(gld[I], da[I], gldda);
+  {
+    // a pair (J, K) at a time, with every use of its raised symbols but Ricci
+    // term 4 (as the FP64 kernel)
+    float dg[18];
+#pragma unroll
+    for (int q = 0; q < 18; ++q) dg[q] = S(S_DG + q);
+#pragma unroll
+    for (int I = 0; I < 3; ++I) Gd[I] = so[I] = 0.f;
 #pragma unroll
     for (int J = 0; J < 3; ++J)
 #pragma unroll
       for (int Kx = J; Kx < 3; ++Kx) {
-        auto dg = [&](int d, int qq) { return S(S_DG + 6 * d + qq); };
-        S(S_G + 6 * I + sym(J, Kx)) =
-            0.5f * (gi[sym(I, 0)] * (dg(J, sym(Kx, 0)) + dg(Kx, sym(J, 0)) - dg(0, sym(J, Kx))) +
-                    gi[sym(I, 1)] * (dg(J, sym(Kx, 1)) + dg(Kx, sym(J, 1)) - dg(1, sym(J, Kx))) +
-                    gi[sym(I, 2)] * (dg(J, sym(Kx, 2)) + dg(Kx, sym(J, 2)) - dg(2, sym(J, Kx))));
-      }
-  {
-    float GLv[3][6];
+        const int q = sym(J, Kx);
+        float b[3], Gq[3];
 #pragma unroll
-    for (int I = 0; I < 3; ++I)
-#pragma unroll
-      for (int J = 0; J < 3; ++J)
-#pragma unroll
-        for (int Kx = J; Kx < 3; ++Kx) {
-          auto dg = [&](int d, int qq) { return S(S_DG + 6 * d + qq); };
-          GLv[I][sym(J, Kx)] = 0.5f * (dg(J, sym(Kx, I)) + dg(Kx, sym(J, I)) - dg(I, sym(J, Kx)));
+        for (int I = 0; I < 3; ++I) {
+          b[I] = 0.5f * (dg[6 * J + sym(Kx, I)] + dg[6 * Kx + sym(J, I)] - dg[6 * I + q]);
+          S(S_DG + 6 * I + q) = b[I];
         }
+        const float wg = J == Kx ? gi[q] : 2.0f * gi[q], wA = J == Kx ? Ac[q] : 2.0f * Ac[q];
 #pragma unroll
-    for (int I = 0; I < 3; ++I)
-#pragma unroll
-      for (int qq = 0; qq < 6; ++qq) S(S_DG + 6 * I + qq) = GLv[I][qq];
+        for (int I = 0; I < 3; ++I) {
+          Gq[I] = dot3f(gi[sym(I, 0)], b[0], gi[sym(I, 1)], b[1], gi[sym(I, 2)], b[2]);
+          Gd[I] = fmaf(Gq[I], wg, Gd[I]);
+          so[I] = fmaf(Gq[I], wA, so[I]);
+        }
+        S(S_DDPHI + q) = S(S_DDPHI + q) - dot3f(Gq[0], dphi[0], Gq[1], dphi[1], Gq[2], dphi[2]);
+        DDa[q] = fmaf(-2.0f, dot3f(dphi[J], da[Kx], dphi[Kx], da[J], -gm[q], gldda),
+                      S(S_DDA + q) - dot3f(Gq[0], da[0], Gq[1], da[1], Gq[2], da[2]));
+      }
   }
-  auto G = [&](int I, int qq) { return S(S_G + 6 * I + qq); };
   auto GL = [&](int I, int qq) { return S(S_DG + 6 * I + qq); };
-  float Gd[3];
+  {
+    const float dKv[3] = {S(S_DK + 0), S(S_DK + 1), S(S_DK + 2)};
+    const float sq[3] = {S(SRC + Q_S1), S(SRC + Q_S2), S(SRC + Q_S3)};
 #pragma unroll
-  for (int I = 0; I < 3; ++I)
-    Gd[I] = G(I, 0) * gi[0] + G(I, 3) * gi[3] + G(I, 5) * gi[5] + 2.0f * (G(I, 1) * gi[1] + G(I, 2) * gi[2] + G(I, 4) * gi[4]);
-  float dphi[3], da[3];
-#pragma unroll
-  for (int d = 0; d < 3; ++d) { dphi[d] = S(S_DPHI + d); da[d] = S(S_DA + d); }
-  float DDa[6], gld[3];
-#pragma unroll
-  for (int I = 0; I < 3; ++I) gld[I] = gi[sym(I, 0)] * dphi[0] + gi[sym(I, 1)] * dphi[1] + gi[sym(I, 2)] * dphi[2];
-#pragma unroll
-  for (int I = 0; I < 3; ++I)
-#pragma unroll
-    for (int J = I; J < 3; ++J) {
-      const int qq = sym(I, J);
-      S(S_DDPHI + qq) = S(S_DDPHI + qq) - (G(0, qq) * dphi[0] + G(1, qq) * dphi[1] + G(2, qq) * dphi[2]);
-      float t = 0.f;
-#pragma unroll
-      for (int L = 0; L < 3; ++L)
-        t += (G(L, qq) + 2.0f * ((L == I ? dphi[J] : 0.f) + (L == J ? dphi[I] : 0.f) - gm[qq] * gld[L])) * da[L];
-      DDa[qq] = S(S_DDA + qq) - t;
+    for (int I = 0; I < 3; ++I) {
+      const float gdK = dot3f(gi[sym(I, 0)], dKv[0], gi[sym(I, 1)], dKv[1], gi[sym(I, 2)], dKv[2]);
+      const float gS = dot3f(gi[sym(I, 0)], sq[0], gi[sym(I, 1)], sq[1], gi[sym(I, 2)], sq[2]);
+      const float s = fmaf(6.0f, dot3f(Ac[sym(I, 0)], dphi[0], Ac[sym(I, 1)], dphi[1], Ac[sym(I, 2)], dphi[2]), so[I]);
+      const float t = dot3f(Ac[sym(I, 0)], da[0], Ac[sym(I, 1)], da[1], Ac[sym(I, 2)], da[2]);
+      S(S_DK + I) = fmaf(2.0f * alpha, fmaf(-8.0f * kPif, gS, fmaf(-2.0f / 3.0f, gdK, s)), -2.0f * t);
     }
+  }
   float DDaTR = gi[0] * DDa[0] + gi[3] * DDa[3] + gi[5] * DDa[5] + 2.0f * (gi[1] * DDa[1] + gi[2] * DDa[2] + gi[4] * DDa[4]);
 #pragma unroll
   for (int m = 0; m < 6; ++m) S(S_DDA + m) = DDa[m] - (1.0f / 3.0f) * gm[m] * DDaTR;
@@ -636,14 +823,27 @@ __device__ __forceinline__ void mixed_body(int nx, int ny, int nz, int lapse, in
   // (about a third of the multiplications; the FP64 kernel keeps the
   // reference's order).
   float t4[6] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
-#pragma unroll
+  // one K at a time in a rolled loop, whose body stays in the instruction
+  // cache; the raised symbols of that K again from the lowered ones
+#pragma unroll 1
   for (int Kx = 0; Kx < 3; ++Kx) {
-    float H[3][3];  // H[M][X]
+    const float r0 = Kx == 0 ? gi[0] : (Kx == 1 ? gi[1] : gi[2]), r1 = Kx == 0 ? gi[1] : (Kx == 1 ? gi[3] : gi[4]),
+                r2 = Kx == 0 ? gi[2] : (Kx == 1 ? gi[4] : gi[5]);
+    const int kq[3] = {Kx, Kx == 0 ? 1 : Kx + 2, Kx == 0 ? 2 : Kx + 3};  // sym(Kx, M)
+    float Gk[6], Gj[3][3], Gl[6], H[3][3];  // Gamma^K_q, Gamma_{J, K M}, Gamma_{K, q}, H[M][X]
+#pragma unroll
+    for (int q = 0; q < 6; ++q) Gk[q] = r0 * GL(0, q) + r1 * GL(1, q) + r2 * GL(2, q);
+#pragma unroll
+    for (int J = 0; J < 3; ++J)
+#pragma unroll
+      for (int M = 0; M < 3; ++M) Gj[J][M] = GL(J, kq[M]);
+#pragma unroll
+    for (int q = 0; q < 6; ++q) Gl[q] = GL(Kx, q);
 #pragma unroll
     for (int M = 0; M < 3; ++M)
 #pragma unroll
       for (int X = 0; X < 3; ++X)
-        H[M][X] = gi[sym(0, M)] * G(Kx, sym(0, X)) + gi[sym(1, M)] * G(Kx, sym(1, X)) + gi[sym(2, M)] * G(Kx, sym(2, X));
+        H[M][X] = gi[sym(0, M)] * Gk[sym(0, X)] + gi[sym(1, M)] * Gk[sym(1, X)] + gi[sym(2, M)] * Gk[sym(2, X)];
 #pragma unroll
     for (int I = 0; I < 3; ++I)
 #pragma unroll
@@ -651,8 +851,8 @@ __device__ __forceinline__ void mixed_body(int nx, int ny, int nz, int lapse, in
         float u = 0.f, w = 0.f;
 #pragma unroll
         for (int M = 0; M < 3; ++M) {
-          u += H[M][I] * GL(J, sym(Kx, M)) + H[M][J] * GL(I, sym(Kx, M));
-          w += H[M][I] * GL(Kx, sym(M, J)) + H[M][J] * GL(Kx, sym(M, I));
+          u += H[M][I] * Gj[J][M] + H[M][J] * Gj[I][M];
+          w += H[M][I] * Gl[sym(M, J)] + H[M][J] * Gl[sym(M, I)];
         }
         t4[sym(I, J)] += u + 0.5f * w;
       }
@@ -662,63 +862,29 @@ __device__ __forceinline__ void mixed_body(int nx, int ny, int nz, int lapse, in
 #pragma unroll
     for (int J = I; J < 3; ++J) {
       const int ij = sym(I, J);
-      auto dGam = [&](int Jx, int Kx) { return S(S_DGAM + 3 * Kx + Jx); };
-      const float t2 = gm[sym(0, I)] * dGam(J, 0) + gm[sym(1, I)] * dGam(J, 1) + gm[sym(2, I)] * dGam(J, 2) +
-                       gm[sym(0, J)] * dGam(I, 0) + gm[sym(1, J)] * dGam(I, 1) + gm[sym(2, J)] * dGam(I, 2);
       const float t3 = Gd[0] * (GL(I, sym(J, 0)) + GL(J, sym(I, 0))) + Gd[1] * (GL(I, sym(J, 1)) + GL(J, sym(I, 1))) +
                        Gd[2] * (GL(I, sym(J, 2)) + GL(J, sym(I, 2)));
-      const float U = -0.5f * S(S_T1 + ij) + 0.5f * t2 + 0.5f * t3 + t4[ij];
+      const float U = S(S_T1 + ij) + 0.5f * t3 + t4[ij];  // terms 1 and 2 were joined in phase 1
       S(S_T1 + ij) = U - 2.0f * (DDphi(ij) - 2.0f * dphi[I] * dphi[J] + gm[ij] * expression);
     }
   auto Ric = [&](int qq) { return S(S_T1 + qq); };
   const float ricci = em4phi * (Ric(0) * gi[0] + Ric(3) * gi[3] + Ric(5) * gi[5] + 2.0f * (Ric(1) * gi[1] + Ric(2) * gi[2] + Ric(4) * gi[4]));
   const float e4phi = __expf(4.0f * phi);
-  float A[6], Ac[6];
-#pragma unroll
-  for (int q = 0; q < 6; ++q) A[q] = D_(F_A11 + q);
-#pragma unroll
-  for (int I = 0; I < 3; ++I)
-#pragma unroll
-    for (int J = I; J < 3; ++J) {
-      float t = 0.f;
-#pragma unroll
-      for (int X = 0; X < 3; ++X)
-#pragma unroll
-        for (int Y = 0; Y < 3; ++Y) t += gi[sym(I, X)] * gi[sym(J, Y)] * A[sym(X, Y)];
-      Ac[sym(I, J)] = t;
-    }
-  const float AijAij = Ac[0] * A[0] + Ac[3] * A[3] + Ac[5] * A[5] + 2.0f * (Ac[1] * A[1] + Ac[2] * A[2] + Ac[4] * A[4]);
 
   // ---- perturbation right-hand sides + FP64 register update ----------------------
-  double outv[NFLD];
   const Taps<true> tko{i, j, k, nx, ny, nz, ny * nz, nz, c};
-  // the RK4 register update (RK4Register.h:180-230) with the substep's
-  // divisors chosen once, one code path per field (as the FP64 kernel's)
-  const double fdiv = stage == 1 ? 6.0 : 3.0, odiv = stage == 3 ? 1.0 : 2.0;
   auto finalize = [&](int fld, float drhs) {
     if constexpr (KO) {
       if (fld < F_D) drhs -= ko_f<O>(a + (size_t)fld * N, tko, (float)bg.ko_scale);
     }
-    const double cv = bgv(bg.rhs, fld) + (double)drhs;
-    const double pv = __ldcs(&P.p[(size_t)fld * N + c]);
-    const double fv = stage == 1 ? 0.0 : __ldcs(&P.f[(size_t)fld * N + c]);
-    const double t = dt * cv;
-    double o;
-    if (stage == 4) {
-      o = fv + (t / 6.0 + pv);
-      __stcs(&P.newp[(size_t)fld * N + c], o);
-    } else {
-      __stcs(&P.f[(size_t)fld * N + c], fv + t / fdiv);
-      o = pv + t / odiv;
-    }
-    outv[fld] = o;
+    S(cvslot(fld)) = drhs;
   };
   // constraint damping (bssn.cc:748-820): H in perturbation form,
   // H - Hbar = -(e^{5 phibar}/8) (expm1(5 dphi) Hcbar + e^{5 dphi} dHc) with
   // dHc = ricci + 2/3 (2 Kbar + dK) dK - A_ij A^ij - 16 pi drho
   float Hd = 0.f, dH = 0.f, dHc = 0.f;
   if (bg.damping) {
-    dHc = ricci + (2.0f / 3.0f) * (2.0f * Kb + dK) * dK - AijAij - 16.0f * kPif * S(S_SRC + Q_R);
+    dHc = ricci + (2.0f / 3.0f) * (2.0f * Kb + dK) * dK - AijAij - 16.0f * kPif * S(SRC + Q_R);
     dH = -(float)(bg.e5phib * (1.0 / 8.0)) * (expm1f(5.0f * dphi0) * (float)bg.Hcbar + __expf(5.0f * dphi0) * dHc);
     Hd = (float)bg.Hbar + dH;
   }
@@ -740,20 +906,13 @@ __device__ __forceinline__ void mixed_body(int nx, int ny, int nz, int lapse, in
 #pragma unroll
         for (int Y = 0; Y < 3; ++Y) aa += gi[sym(X, Y)] * A[sym(X, I)] * A[sym(Y, J)];
       const float RTF = Ric(qq) - (1.0f / 3.0f) * e4phi * gm[qq] * ricci;
-      float v = em4phi * (alpha * (RTF - 8.0f * kPif * S(S_SRC + Q_STF11 + qq)) - S(S_DDA + qq)) +
+      float v = em4phi * (alpha * (RTF - 8.0f * kPif * S(SRC + Q_STF11 + qq)) - S(S_DDA + qq)) +
                 alpha * (K * A[qq] - 2.0f * aa);
       if (bg.damping) v -= adt * A[qq] * Hd;
       finalize(F_A11 + qq, v);
     }
 #pragma unroll
-  for (int I = 0; I < 3; ++I) {
-    const float so = G(I, 0) * Ac[0] + G(I, 3) * Ac[3] + G(I, 5) * Ac[5] + 2.0f * (G(I, 1) * Ac[1] + G(I, 2) * Ac[2] + G(I, 4) * Ac[4]) +
-                     6.0f * (Ac[sym(I, 0)] * dphi[0] + Ac[sym(I, 1)] * dphi[1] + Ac[sym(I, 2)] * dphi[2]);
-    const float gdK = gi[sym(I, 0)] * S(S_DK + 0) + gi[sym(I, 1)] * S(S_DK + 1) + gi[sym(I, 2)] * S(S_DK + 2);
-    const float gS = gi[sym(I, 0)] * S(S_SRC + Q_S1) + gi[sym(I, 1)] * S(S_SRC + Q_S2) + gi[sym(I, 2)] * S(S_SRC + Q_S3);
-    finalize(F_GAM1 + I, -2.0f * (Ac[sym(I, 0)] * da[0] + Ac[sym(I, 1)] * da[1] + Ac[sym(I, 2)] * da[2]) +
-                             2.0f * alpha * (so - (2.0f / 3.0f) * gdK - 8.0f * kPif * gS));
-  }
+  for (int I = 0; I < 3; ++I) finalize(F_GAM1 + I, S(S_DK + I));
   // zeroth-order equations in explicit perturbation form
   const float dRK = -DDaTR + (alb * (2.0f * Kb + dK) * dK + dal * K * K) * (1.0f / 3.0f) + alpha * AijAij +
                     4.0f * kPif * (alb * (dr + Sdust) + dal * rS_full);
@@ -761,27 +920,64 @@ __device__ __forceinline__ void mixed_body(int nx, int ny, int nz, int lapse, in
   finalize(F_PHI, bg.damping ? -(1.0f / 6.0f) * (alb * dK + dal * K) + 0.1f * adt * dH
                              : -(1.0f / 6.0f) * (alb * dK + dal * K));
   finalize(F_ALPHA, lapse_drhs(lapse, bg, alb, dal, alpha, Kb, dK, dphi0, P.kavg ? (float)__ldg(P.kavg) : 0.0f));
-  if (MATTER == kDust) {
-#pragma unroll
-    for (int m = 0; m < 4; ++m) finalize(F_D + m, rhs_m[m]);
-  } else if (MATTER == kScalar) {
-#pragma unroll
-    for (int m = 0; m < 5; ++m) finalize(F_SPHI + m, rhs_m[m]);
-  }
 
-  if (stage == 4) {
-    bool bad_any = false;
+  // the RK4 register update (RK4Register.h:180-230) of every field, one rolled
+  // loop, the registers of eight fields loaded at once; the substep's factors chosen once: f = f + dt cv / 6 (substep 1, from f = 0),
+  // / 3 (2, 3); a = p + dt cv / 2 (1, 2), / 1 (3); p = f + (dt cv / 6 + p) (4).
+  // The new values (FP32) replace the right-hand sides in the slots; at the
+  // last substep g and A, which are normalised below, stay in FP64 too.
+  const bool renorm = stage == 4 && normalize;
+  bool bad_any = false, bad_phi = false;
+  const double wf = dt * (stage == 1 || stage == 4 ? 1.0 / 6.0 : 1.0 / 3.0), wo = stage == 3 ? dt : 0.5 * dt;
+  auto update = [&](auto last) {
+    constexpr bool kLast = decltype(last)::value;
+    constexpr int CH = 8;
+#pragma unroll 1
+    for (int f0 = 0; f0 < NFLD; f0 += CH) {
+      double pv[CH], fv[CH];
 #pragma unroll
-    for (int f = 0; f < NFLD; ++f) bad_any |= !isfinite(outv[f]);
-    if (bad_any) {
-      if (isnan(outv[F_PHI])) atomicOr(P.status, 1u);
-      atomicOr(P.status, 2u);
+      for (int q = 0; q < CH; ++q) {
+        if (f0 + q >= NFLD) continue;
+        pv[q] = __ldcs(fat(P.p, f0 + q));
+        fv[q] = !kLast && stage == 1 ? 0.0 : __ldcs(fat(P.f, f0 + q));
+      }
+#pragma unroll
+      for (int q = 0; q < CH; ++q) {
+        const int fld = f0 + q;
+        if (fld >= NFLD) continue;
+        const double cv = bg_rhs[fld] + (double)S(cvslot(fld));
+        const double f1 = fv[q] + wf * cv;
+        const double o = kLast ? f1 + pv[q] : pv[q] + wo * cv;
+        __stcs(fat(kLast ? P.newp : P.f, fld), kLast ? o : f1);
+        S(cvslot(fld)) = (float)o;
+        if constexpr (kLast) {
+          bad_any |= !isfinite(o);
+          if (fld == F_PHI) bad_phi = isnan(o);
+          if (renorm && fld < F_K && fld != F_PHI) {
+            const int s = S_WIDE + 2 * (fld < F_PHI ? fld : fld - F_A11 + 6);
+            S(s) = __int_as_float(__double2loint(o));
+            S(s + 1) = __int_as_float(__double2hiint(o));
+            continue;
+          }
+        }
+        __stcs(fat(P.out, fld), (float)(o - bg_out[fld]));
+      }
     }
+  };
+  if (stage == 4) update(std::true_type());
+  else update(std::false_type());
+  if (bad_any) {
+    if (bad_phi) atomicOr(P.status, 1u);
+    atomicOr(P.status, 2u);
+  }
+  if (renorm) {
     // the next step's first-substep input is the normalised new state (bssn.cc:224-225)
-    if (normalize) {
+    auto wide = [&](int q) {
+      return __hiloint2double(__float_as_int(S(S_WIDE + 2 * q + 1)), __float_as_int(S(S_WIDE + 2 * q)));
+    };
     double gn[6], An[6];
 #pragma unroll
-    for (int m = 0; m < 6; ++m) { gn[m] = outv[F_G11 + m]; An[m] = outv[F_A11 + m]; }
+    for (int m = 0; m < 6; ++m) { gn[m] = wide(m); An[m] = wide(6 + m); }
     {
       double omd = -1.0 * (gn[0] + gn[3] + gn[5] - gn[1] * gn[1] - gn[2] * gn[2] - gn[4] * gn[4] + gn[0] * gn[3] +
                            gn[0] * gn[5] + gn[3] * gn[5] - gn[4] * gn[4] * gn[0] - gn[2] * gn[2] * gn[3] -
@@ -806,34 +1002,35 @@ __device__ __forceinline__ void mixed_body(int nx, int ny, int nz, int lapse, in
       An[4] = (An[4] - 1.0 / 3.0 * gn[4] * trA) * inv;
     }
 #pragma unroll
-    for (int m = 0; m < 6; ++m) { outv[F_G11 + m] = gn[m]; outv[F_A11 + m] = An[m]; }
+    for (int m = 0; m < 6; ++m) {
+      S(cvslot(F_G11 + m)) = (float)gn[m];
+      __stcs(fat(P.out, F_G11 + m), (float)gn[m]);
+      __stcs(fat(P.out, F_A11 + m), (float)An[m]);
     }
   }
-#pragma unroll
-  for (int f = 0; f < NFLD; ++f) __stcs(&P.out[(size_t)f * N + c], (float)(outv[f] - bgv(bg.out, f)));
   if (MATTER == kDust) {
     float go[6], gio[6];
 #pragma unroll
-    for (int m = 0; m < 6; ++m) go[m] = (float)outv[F_G11 + m];
+    for (int m = 0; m < 6; ++m) go[m] = S(cvslot(F_G11 + m));
     inv_metricf(go, gio);
-    const float So[3] = {(float)outv[F_S1], (float)outv[F_S2], (float)outv[F_S3]};
-    const float phio = (float)outv[F_PHI];
-    const float Do = (float)outv[F_D];
+    const float So[3] = {S(cvslot(F_S1)), S(cvslot(F_S2)), S(cvslot(F_S3))};
+    const float phio = S(cvslot(F_PHI));
+    const float Do = S(cvslot(F_D));
     const DustF dp = dust_primf(gio, __expf(-4.0f * phio), __expf(6.0f * phio), Do, So);
-    const float alo = (float)(outv[F_ALPHA] + 1.0);
+    const float alo = S(cvslot(F_ALPHA)) + 1.0f;
     float* fo = P.fp_out;
-    __stcs(&fo[(size_t)P_AD * N + c], alo * Do);
+    __stcs(fat(fo, P_AD), alo * Do);
 #pragma unroll
-    for (int m = 0; m < 3; ++m) __stcs(&fo[(size_t)(P_AS1 + m) * N + c], alo * So[m]);
+    for (int m = 0; m < 3; ++m) __stcs(fat(fo, P_AS1 + m), alo * So[m]);
 #pragma unroll
-    for (int m = 0; m < 3; ++m) __stcs(&fo[(size_t)(P_V1 + m) * N + c], dp.v[m]);
+    for (int m = 0; m < 3; ++m) __stcs(fat(fo, P_V1 + m), dp.v[m]);
   }
 }
 
-// the TMA barrier of a CTA: initialised once, before any copy
-__device__ __forceinline__ void init_tile_barrier(uint64_t* bar, bool use) {
+// the TMA barriers of a CTA: initialised once, before any copy
+__device__ __forceinline__ void init_tile_barriers(uint64_t* bar, bool use) {
   if (use && threadIdx.x == 0 && threadIdx.y == 0 && threadIdx.z == 0) {
-    tma::bar_init(bar, 1);
+    for (int b = 0; b < 3; ++b) tma::bar_init(bar + b, 1);
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
   __syncthreads();
@@ -842,16 +1039,17 @@ __device__ __forceinline__ void init_tile_barrier(uint64_t* bar, bool use) {
 // One box: one CTA per updated brick.  tmap: the TMA map of this substep's
 // input (use_tma = 0: every tile is copied by the threads).
 template <int O, int MATTER, bool KO>
-__global__ void __launch_bounds__(kThreads, 4)
+__global__ void __launch_bounds__(kThreads, (Layout<O, MATTER>::CTAS))
 mixed_kernel(int nx, int ny, int nz, int lapse, int normalize, float idx, double dt, Bg bg, Ptrs P, int stage,
-             const __grid_constant__ CUtensorMap tmap, int use_tma, int bx0) {
-  __shared__ __align__(8) uint64_t bar;
-  init_tile_barrier(&bar, use_tma != 0);
+             const __grid_constant__ CUtensorMap tmap, int use_tma, int bx0, const __grid_constant__ FluxMaps fmaps,
+             int use_fmaps) {
+  __shared__ __align__(8) uint64_t bar[3];
+  init_tile_barriers(bar, use_tma != 0);
   unsigned phase = 0;
   bool tma_ok = true;
   // bx0: first x brick (x-slab boxes skip their ghost planes)
   mixed_body<O, MATTER, KO>(nx, ny, nz, lapse, normalize, idx, dt, bg, P, stage, blockIdx.z + bx0, blockIdx.y, blockIdx.x,
-                        use_tma ? &tmap : nullptr, &bar, phase, tma_ok);
+                        use_tma ? &tmap : nullptr, bar, phase, tma_ok, use_tma && use_fmaps ? &fmaps : nullptr);
 }
 
 // Register roles of substep n (X/Y ping-pong, as in the single-box launcher).
@@ -874,15 +1072,16 @@ __device__ __forceinline__ Ptrs group_ptrs(const GroupBox& b, int stage) {
 // A group of mixed boxes, one launch per substep over the work list of all
 // their bricks (see the FP64 stage_group_kernel).
 template <int O, int MATTER>
-__global__ void __launch_bounds__(kThreads, 4)
+__global__ void __launch_bounds__(kThreads, (Layout<O, MATTER>::CTAS))
 mixed_group_kernel(const GroupBox* __restrict__ boxes, GroupBg gb, int stage) {
   __shared__ GroupBox sb;
   __shared__ Ptrs sp;
   __shared__ Bg sbg;
   __shared__ const CUtensorMap* stm;
-  __shared__ __align__(8) uint64_t bar;
+  __shared__ const FluxMaps* sfm;
+  __shared__ __align__(8) uint64_t bar[3];
   const bool lead = threadIdx.x == 0 && threadIdx.y == 0 && threadIdx.z == 0;
-  init_tile_barrier(&bar, true);
+  init_tile_barriers(bar, true);
   unsigned phase = 0;
   bool tma_ok = true;
   for (int w = blockIdx.x; w < gb.total; w += gridDim.x) {
@@ -899,12 +1098,20 @@ mixed_group_kernel(const GroupBox* __restrict__ boxes, GroupBg gb, int stage) {
       // the map is read from global memory (a TMA map cannot live in shared memory)
       stm = boxes[lo].tma ? (stage == 1 || stage == 3 ? &boxes[lo].mapX : &boxes[lo].mapY) : nullptr;
       if (stm) tma::acquire_map(stm);  // the host wrote the map into the table
+      sfm = nullptr;
+      if (MATTER == kDust && stm) {  // the flux-primitive boxes, after the GroupBox entries
+        const GroupFluxMaps& fx = reinterpret_cast<const GroupFluxMaps*>(boxes + gb.nboxes)[lo];
+        if (fx.valid) {
+          sfm = reinterpret_cast<const FluxMaps*>(stage == 1 || stage == 3 ? fx.fp0 : fx.fp1);
+          for (int a = 0; a < 3; ++a) tma::acquire_map(&sfm->m[a]);
+        }
+      }
     }
     __syncthreads();
     const int l = w - sb.first;
     const int cz = l % sb.nbz, cy = (l / sb.nbz) % sb.nby, cx = l / (sb.nbz * sb.nby);
     mixed_body<O, MATTER>(sb.nx, sb.ny, sb.nz, sb.lapse, sb.normalize, sb.idx, sb.dt, sbg, sp, stage, cx, cy, cz, stm,
-                          &bar, phase, tma_ok);
+                          bar, phase, tma_ok, sfm);
   }
 }
 

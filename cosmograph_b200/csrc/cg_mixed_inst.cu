@@ -10,13 +10,8 @@ namespace mixed {
 namespace {
 dim3 grid3(int nx, int ny, int nz) { return dim3((nz + kBZ - 1) / kBZ, (ny + kBY - 1) / kBY, (nx + kBX - 1) / kBX); }
 
-template <int M>
-constexpr size_t smem_bytes() {
-  return sizeof(float) * NSlot<M>::value * kThreads;
-}
-
-// dynamic shared memory above the 48 KB default (the scalar slots) needs
-// the kernel's attribute raised once
+// dynamic shared memory above the 48 KB default needs the kernel's attribute
+// raised once
 template <class K>
 cudaError_t allow_smem(K kernel, size_t smem, bool& done) {
   if (done || smem <= 48 * 1024) return cudaSuccess;
@@ -39,13 +34,16 @@ cudaError_t go(const MixedBox& b, const Bg& bg, int stage, cudaStream_t st) {
     case 3: P.in = b.X; P.prev = b.Y; P.out = b.Y; P.fp_in = b.FP0; P.fp_out = b.FP1; break;
     default: P.in = b.Y; P.prev = b.X; P.out = b.X; P.fp_in = b.FP1; P.fp_out = b.FP0; break;
   }
-  constexpr size_t smem = smem_bytes<M>();
+  constexpr size_t smem = Layout<O, M>::kBytes;
   static bool done = false;
   cudaError_t e = allow_smem(mixed_kernel<O, M, KO>, smem, done);
   if (e != cudaSuccess) return e;
   const CUtensorMap& map = (stage == 1 || stage == 3) ? b.mapX : b.mapY;  // the substep's input
+  FluxMaps fm;
+  for (int q = 0; q < 3; ++q) fm.m[q] = (stage == 1 || stage == 3) ? b.fmap0[q] : b.fmap1[q];
   mixed_kernel<O, M, KO><<<grid3(b.nx - 2 * b.xg, b.ny, b.nz), dim3(kBZ, kBY, kBX), smem, st>>>(
-      b.nx, b.ny, b.nz, b.lapse, b.normalize, (float)(1.0 / b.dx), b.dt, bg, P, stage, map, b.tma, b.xg / kBX);
+      b.nx, b.ny, b.nz, b.lapse, b.normalize, (float)(1.0 / b.dx), b.dt, bg, P, stage, map, b.tma, b.xg / kBX, fm,
+      b.fmaps);
   return cudaGetLastError();
 }
 template <int O, bool KO>
@@ -67,7 +65,7 @@ cudaError_t go_m(const MixedBox& b, const Bg& bg, int stage, cudaStream_t st) {
 
 template <int O, int M>
 cudaError_t go_group(const GroupBox* table, const GroupBg& gb, int stage, int grid, cudaStream_t st) {
-  constexpr size_t smem = smem_bytes<M>();
+  constexpr size_t smem = Layout<O, M>::kBytes;
   static bool done = false;
   cudaError_t e = allow_smem(mixed_group_kernel<O, M>, smem, done);
   if (e != cudaSuccess) return e;
@@ -85,7 +83,7 @@ cudaError_t go_group_m(const GroupBox* table, const GroupBg& gb, int matter, int
 }
 template <int O, int M>
 int ctas() {
-  constexpr size_t smem = smem_bytes<M>();
+  constexpr size_t smem = Layout<O, M>::kBytes;
   static bool done = false;
   if (allow_smem(mixed_group_kernel<O, M>, smem, done) != cudaSuccess) return 1;
   int n = 0;
@@ -104,15 +102,28 @@ int ctas_m(int matter) {
 template <int O>
 bool encode_maps(MixedBox& b) {
   using G = TileG<O>;
-  return tma_host::encode(&b.mapX, b.X, sizeof(float), b.nx, b.ny, b.nz, b.nfields, G::TZ, G::TY, G::TX) &&
-         tma_host::encode(&b.mapY, b.Y, sizeof(float), b.nx, b.ny, b.nz, b.nfields, G::TZ, G::TY, G::TX);
+  if (!(tma_host::encode(&b.mapX, b.X, sizeof(float), b.nx, b.ny, b.nz, b.nfields, G::TZ, G::TY, G::TX) &&
+        tma_host::encode(&b.mapY, b.Y, sizeof(float), b.nx, b.ny, b.nz, b.nfields, G::TZ, G::TY, G::TX)))
+    return false;
+  if (b.FP0 && b.FP1) {  // dust: x, y, z boxes of the flux primitives
+    const int box[3][3] = {{kBZ, kBY, kBX + O}, {kBZ, kBY + O, kBX}, {G::TZ, kBY, kBX}};
+    bool ok = true;
+    for (int a = 0; a < 3; ++a) {
+      ok = ok && tma_host::encode(&b.fmap0[a], b.FP0, sizeof(float), b.nx, b.ny, b.nz, P_N, box[a][0], box[a][1], box[a][2]);
+      ok = ok && tma_host::encode(&b.fmap1[a], b.FP1, sizeof(float), b.nx, b.ny, b.nz, P_N, box[a][0], box[a][1], box[a][2]);
+    }
+    b.fmaps = ok ? 1 : 0;
+  }
+  return true;
 }
 }  // namespace
 
 void make_tile_maps(MixedBox& b) {
   std::memset(&b.mapX, 0, sizeof(b.mapX));
   std::memset(&b.mapY, 0, sizeof(b.mapY));
-  b.maps = b.tma = 0;
+  std::memset(b.fmap0, 0, sizeof(b.fmap0));
+  std::memset(b.fmap1, 0, sizeof(b.fmap1));
+  b.maps = b.tma = b.fmaps = 0;
   // row strides must be multiples of 16 bytes; the bases are cudaMalloc'd
   if (b.nz % 4 != 0 || !b.X || !b.Y) return;
   bool ok = false;

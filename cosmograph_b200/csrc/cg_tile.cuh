@@ -28,7 +28,7 @@ struct Brick {
   static constexpr int BX = BX_, BY = BY_, BZ = BZ_, THREADS = BX * BY * BZ, WARPS = THREADS / 32;
 };
 using Brick64 = Brick<4, 6, 16>;
-using Brick32 = Brick<4, 4, 8>;
+using Brick32 = Brick<4, 8, 8>;
 
 // PITCH: row pitch in elements (0: the copied row length).  ZOFF: tile
 // column 0 holds z = z0 - ZOFF (default r); the copy fills columns
@@ -69,36 +69,6 @@ __device__ __forceinline__ void row_offsets(int x0, int y0, int nx, int ny, int 
     rowoff[r] = (x * ny + y) * nz;
   }
 }
-
-// Copy of one field's tile.  Lane l of warp w works on column z = l mod TZU of
-// row (w + WARPS*q)*RPP + l / TZU at step q.  fetch() issues the global loads
-// into registers, store() writes them to the tile.
-template <class G, class B, class T>
-struct Loader {
-  T buf[G::NPW];
-  int row0, col, zoff;  // zoff < 0: lane without a column
-  __device__ __forceinline__ void init(int tid, int z0, int nz) {
-    const int warp = tid >> 5, lane = tid & 31;
-    const int sub = lane / G::TZU;
-    col = lane - sub * G::TZU;
-    row0 = warp * G::RPP + sub;
-    zoff = sub < G::RPP ? pmod(z0 - G::R + col, nz) : -1;
-  }
-  __device__ __forceinline__ void fetch(const T* __restrict__ f, const int* rowoff) {
-#pragma unroll
-    for (int q = 0; q < G::NPW; ++q) {
-      const int r = row0 + B::WARPS * G::RPP * q;
-      if (zoff >= 0 && r < G::ROWS) buf[q] = __ldg(f + rowoff[r] + zoff);
-    }
-  }
-  __device__ __forceinline__ void store(T* tl) const {
-#pragma unroll
-    for (int q = 0; q < G::NPW; ++q) {
-      const int r = row0 + B::WARPS * G::RPP * q;
-      if (zoff >= 0 && r < G::ROWS) tl[r * G::TZ + G::CO + col] = buf[q];
-    }
-  }
-};
 
 // Asynchronous copy of one field's tile (cp.async, global to shared memory,
 // no register staging).  Lane l of warp w copies column z = l mod TZU of row
