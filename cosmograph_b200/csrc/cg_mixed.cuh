@@ -124,6 +124,12 @@ struct FluxBox {
 struct FluxMaps {
   CUtensorMap m[3];  // x, y and z boxes of the substep input's 7 flux-primitive arrays
 };
+// Bricks of 4 x 4 x 16 points, two CTAs per SM.  What bounds the kernel is the
+// memory system at the granularity of a brick's rows (a substep touches some 60
+// arrays): rows of 16 points instead of 8 make every register row a whole
+// 128-byte line, and the 24-float row of a field tile holds no unused columns.
+// ms a step, 256^3 dust / 128^3 scalar, order 8: 4 x 4 x 8 with four CTAs 28.6 /
+// 4.06, 4 x 8 x 8 with two 26.1 / 3.52, 4 x 4 x 16 with two 24.3 / 3.01.
 // Shared memory of a CTA, in floats: phase 1 the slots that survive it, then
 // the field tiles (two where CTAS CTAs per SM still fit); the flux boxes lie
 // over the still empty slots.  Phase 2: the sources take the tiles' place.
@@ -382,7 +388,7 @@ __device__ __forceinline__ bool derivatives(const float* __restrict__ a, int N, 
     if (tid == 0) {
       tma::arrive_expect_tx(bar + b, (unsigned)(G::SIZE * sizeof(float)));
       tma::load_4d(b ? tl2 : tl, tmap, z0 - G::ZO, y0 - G::R, x0 - G::R, PF::field(it), bar + b);
-      if (it + 1 < PF::N) tma::prefetch_4d(tmap, z0 - G::ZO, y0 - G::R, x0 - G::R, PF::field(it + 1));
+      if (!TWO && it + 1 < PF::N) tma::prefetch_4d(tmap, z0 - G::ZO, y0 - G::R, x0 - G::R, PF::field(it + 1));
     }
     pending |= 1u << b;
   };
@@ -534,7 +540,11 @@ __device__ __forceinline__ void mixed_body(int nx, int ny, int nz, int lapse, in
   float* sl = smf + L::MATN * kThreads + tid;  // this thread's slot column
   auto S = [&](int s) -> float& { return sl[s * kThreads]; };
   const int k0 = cz * kBZ + threadIdx.x;
-  const int j0 = cy * kBY + threadIdx.y;
+  // the two 16-point rows of a warp lie two y apart: two tile rows of 24 floats
+  // are 16 banks, so a warp's tap takes one wavefront
+  static_assert(kBY == 4 && kBZ == 16, "row pairs of a warp");
+  const int ty = (threadIdx.y & 1) << 1 | threadIdx.y >> 1;
+  const int j0 = cy * kBY + ty;
   const int i0 = cx * kBX + threadIdx.z;
   // every thread takes part in the tile copies; threads past the box edge
   // compute a valid point and leave after phase 1
@@ -593,7 +603,7 @@ __device__ __forceinline__ void mixed_body(int nx, int ny, int nz, int lapse, in
     }
     flux_tiles = L::FLUX && fmaps && by_tma;
     // after a copy timed out the CTA copies by threads (the barrier's phase is unknown)
-    tma_ok = derivatives<O, MATTER>(a, N, idx, idx2, g, gi, smf, sl, tid, x0, y0, z0, threadIdx.z, threadIdx.y,
+    tma_ok = derivatives<O, MATTER>(a, N, idx, idx2, g, gi, smf, sl, tid, x0, y0, z0, threadIdx.z, ty,
                                     threadIdx.x, nz, by_tma ? tmap : nullptr, flux_tiles ? fmaps : nullptr, bar,
                                     phase, P.status, bg.tma_wait) && tma_ok;
     __syncthreads();  // the tiles become slots again

@@ -11,9 +11,9 @@
 // conflicts:
 //   FP64, 16 points along z: a warp reads two contiguous 16-double rows (two
 //         wavefronts, the minimum for 256 bytes);
-//   FP32, 8 points along z with a row pitch of 24 floats: a warp reads four
-//         8-float row segments whose banks are s, s+24, s+16, s+8 (mod 32),
-//         one wavefront.
+//   FP32, 16 points along z with a row pitch of 24 floats: a warp reads two
+//         16-float row segments; the kernel pairs rows two y apart, whose
+//         banks are s and s+16 (mod 32), one wavefront.
 //
 // The copies run asynchronously (cp.async, AsyncLoader, or TMA boxes): the
 // next field's into a second tile buffer where there is one, else while the
@@ -28,7 +28,7 @@ struct Brick {
   static constexpr int BX = BX_, BY = BY_, BZ = BZ_, THREADS = BX * BY * BZ, WARPS = THREADS / 32;
 };
 using Brick64 = Brick<4, 6, 16>;
-using Brick32 = Brick<4, 8, 8>;
+using Brick32 = Brick<4, 4, 16>;
 
 // PITCH: row pitch in elements (0: the copied row length).  ZOFF: tile
 // column 0 holds z = z0 - ZOFF (default r); the copy fills columns
@@ -46,8 +46,6 @@ struct Geom {
   static constexpr int ROWS = TX * TY;
   static constexpr int SIZE = ROWS * TZ;
   static constexpr int SY = TZ, SX = TY * TZ;
-  static constexpr int RPP = 32 / TZU;                    // rows per warp instruction
-  static constexpr int NPW = (ROWS + B::WARPS * RPP - 1) / (B::WARPS * RPP);  // instructions per warp
   static_assert(TZU <= 32, "one warp copies at least one tile row");
 };
 
@@ -71,9 +69,9 @@ __device__ __forceinline__ void row_offsets(int x0, int y0, int nx, int ny, int 
 }
 
 // Asynchronous copy of one field's tile (cp.async, global to shared memory,
-// no register staging).  Lane l of warp w copies column z = l mod TZU of row
-// (w + WARPS*q)*RPP + l / TZU at step q.  issue() starts this thread's copies
-// and commits them as one group; the caller waits for its groups
+// no register staging).  Lane l of warp w copies group l mod GROUPS of row
+// (w + WARPS*q)*RPP + l / GROUPS at step q.  issue() starts this thread's
+// copies and commits them as one group; the caller waits for its groups
 // (cp_async_wait) and synchronises the CTA before reading.
 template <int BYTES>
 __device__ __forceinline__ void cp_async(void* dst, const void* src) {
@@ -87,43 +85,51 @@ __device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commi
 template <int N>
 __device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory"); }
 
-// Whole 16-byte groups where every row starts on 16 bytes (nz a multiple of
-// V = 16 / sizeof(T)): the tile's rows then hold whole groups from the aligned
-// column 0 on, and a group never straddles the periodic wrap; a quarter
-// (FP32) or half (FP64) of the instructions.
+// Groups of W = 16 / sizeof(T) elements where every row starts on 16 bytes (nz
+// a multiple of W), of W / 2 where it starts on half of that, else single
+// elements: the tile's rows then hold whole groups from the aligned column 0
+// on, and a group never straddles the periodic wrap.
 template <class G, class B, class T>
 struct AsyncLoader {
-  static constexpr int V = 16 / (int)sizeof(T);
-  static constexpr int C0 = G::CO / V * V;                      // first copied column of the wide form
-  static constexpr int GROUPS = (G::CO + G::TZU - C0 + V - 1) / V;  // groups per row
-  static constexpr int RPPW = 32 / GROUPS;
-  static constexpr int NPWW = (G::ROWS + B::WARPS * RPPW - 1) / (B::WARPS * RPPW);
-  static_assert(C0 + GROUPS * V <= G::TZ && G::TZ % V == 0 && G::ZO % V == 0, "whole groups stay inside a row");
+  static constexpr int W = 16 / (int)sizeof(T);
+  // the copy in groups of V elements
+  template <int V>
+  struct Form {
+    static constexpr int C0 = G::CO / V * V;                          // first copied column
+    static constexpr int GROUPS = (G::CO + G::TZU - C0 + V - 1) / V;  // groups per row
+    static constexpr int RPP = 32 / GROUPS;                           // rows per warp instruction
+    static constexpr int NPW = (G::ROWS + B::WARPS * RPP - 1) / (B::WARPS * RPP);
+    static_assert(C0 + GROUPS * V <= G::TZ && G::TZ % V == 0 && G::ZO % V == 0, "whole groups stay inside a row");
+  };
   int row0, col, zoff;  // zoff < 0: lane without a column
-  bool wide;
+  int form;             // elements per group
+  template <int V>
+  __device__ __forceinline__ void init_form(int tid, int z0, int nz) {
+    using F = Form<V>;
+    const int warp = tid >> 5, lane = tid & 31, sub = lane / F::GROUPS;
+    form = V;
+    col = F::C0 + (lane - sub * F::GROUPS) * V;
+    row0 = warp * F::RPP + sub;
+    zoff = sub < F::RPP ? pmod(z0 - G::ZO + col, nz) : -1;
+  }
   __device__ __forceinline__ void init(int tid, int z0, int nz) {
-    const int warp = tid >> 5, lane = tid & 31;
-    wide = nz % V == 0;
-    const int per = wide ? GROUPS : G::TZU, rpp = wide ? RPPW : G::RPP;
-    const int sub = lane / per;
-    col = wide ? C0 + (lane - sub * per) * V : G::CO + lane - sub * per;
-    row0 = warp * rpp + sub;
-    zoff = sub < rpp ? pmod(z0 - G::ZO + col, nz) : -1;
+    if (nz % W == 0) init_form<W>(tid, z0, nz);
+    else if (W > 2 && nz % (W / 2) == 0) init_form<(W > 2 ? W / 2 : 1)>(tid, z0, nz);
+    else init_form<1>(tid, z0, nz);
+  }
+  template <int V>
+  __device__ __forceinline__ void issue_form(T* tl, const T* __restrict__ f, const int* rowoff) const {
+    using F = Form<V>;
+#pragma unroll
+    for (int q = 0; q < F::NPW; ++q) {
+      const int r = row0 + B::WARPS * F::RPP * q;
+      if (zoff >= 0 && r < G::ROWS) cp_async<V * (int)sizeof(T)>(tl + r * G::TZ + col, f + rowoff[r] + zoff);
+    }
   }
   __device__ __forceinline__ void issue(T* tl, const T* __restrict__ f, const int* rowoff) const {
-    if (wide) {
-#pragma unroll
-      for (int q = 0; q < NPWW; ++q) {
-        const int r = row0 + B::WARPS * RPPW * q;
-        if (zoff >= 0 && r < G::ROWS) cp_async<16>(tl + r * G::TZ + col, f + rowoff[r] + zoff);
-      }
-    } else {
-#pragma unroll
-      for (int q = 0; q < G::NPW; ++q) {
-        const int r = row0 + B::WARPS * G::RPP * q;
-        if (zoff >= 0 && r < G::ROWS) cp_async<(int)sizeof(T)>(tl + r * G::TZ + col, f + rowoff[r] + zoff);
-      }
-    }
+    if (form == W) issue_form<W>(tl, f, rowoff);
+    else if (W > 2 && form == W / 2) issue_form<(W > 2 ? W / 2 : 1)>(tl, f, rowoff);
+    else issue_form<1>(tl, f, rowoff);
     cp_async_commit();
   }
 };

@@ -1,4 +1,4 @@
-"""Boxes at the edges of the kernels' bricks (FP64 4 x 6 x 16, mixed 4 x 8 x 8
+"""Boxes at the edges of the kernels' bricks (FP64 4 x 6 x 16, mixed 4 x 4 x 16
 points of x, y, z): one brick, one point more, whole bricks only, bricks away
 from every face (TMA tiles and flux boxes), odd and even row lengths (wide and
 narrow thread copies).  FP64 bit for bit against the restatement with correctly
@@ -28,7 +28,7 @@ def test_fp64_brick_edges_bit_exact(case, order):
 
 
 @pytest.mark.parametrize("order", [2, 4, 6, 8])
-@pytest.mark.parametrize("shape", [(5, 8, 8), (8, 9, 10), (12, 16, 16), (13, 25, 28)])
+@pytest.mark.parametrize("shape", [(5, 8, 16), (8, 9, 18), (13, 5, 17), (12, 12, 48), (13, 18, 20)])
 def test_mixed_brick_edges(shape, order):
     """FP32 perturbations of amplitude 1e-3, one step of dt = 0.1 dx: second
     differences carry 2^-24 / dx^2 relative to the perturbation and enter with
